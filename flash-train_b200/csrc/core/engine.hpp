@@ -171,7 +171,9 @@ class OpsEngine final : public OpsEngineBase {
                 throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "Applicable Primitive returned a null clone");
             }
             static_cast<Primitive<Problem>&>(*copy).configure(problem);
+            std::unique_ptr<PrimitiveBase> lean = copy->cloneForMinimumWorkspace();
             primitives.push_back(std::move(copy));
+            if (lean != nullptr) { primitives.push_back(std::move(lean)); }
         }
         return primitives;
     }

@@ -5,7 +5,7 @@ namespace ftrain {
 PrimitiveBase::~PrimitiveBase() = default;
 
 void PrimitiveBase::execute(const Resources& resources) {
-    const std::uint64_t required = getRequiredWorkspaceBytes();
+    const std::uint64_t required = getMinimumWorkspaceBytes();
     if (resources.getWorkspaceBytes() < required) {
         throw Exception(FTRAIN_STATUS_INVALID_ARGUMENT, "the workspace holds %llu bytes; this Primitive needs %llu",
                         static_cast<unsigned long long>(resources.getWorkspaceBytes()),

@@ -37,11 +37,16 @@ struct PrimitiveBase {
     // FTRAIN_ENABLED_PRIMITIVES / FTRAIN_DISABLED_PRIMITIVES.
     virtual const char* getName() const noexcept = 0;
     virtual std::unique_ptr<PrimitiveBase> clone() const = 0;
-    // Meaningful after configure().
+    // Meaningful after configure(). What the Primitive's best form uses.
     virtual std::uint64_t getRequiredWorkspaceBytes() const noexcept = 0;
+    // What it cannot do without: a Primitive may have a form that does with less.
+    virtual std::uint64_t getMinimumWorkspaceBytes() const noexcept { return getRequiredWorkspaceBytes(); }
+    // A configured Primitive whose best form uses more than the minimum: a copy kept to the
+    // minimum, which follows it in the Plan for callers that walk the indices by workspace budget. Else null.
+    virtual std::unique_ptr<PrimitiveBase> cloneForMinimumWorkspace() const { return nullptr; }
 
     // Throws Exception(FTRAIN_STATUS_INVALID_ARGUMENT), without dispatching,
-    // when the workspace is smaller than required or null while required.
+    // when the workspace is smaller than the minimum or null while one is needed.
     void execute(const Resources& resources);
 
   protected:

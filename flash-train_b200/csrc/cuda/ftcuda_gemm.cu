@@ -12,6 +12,15 @@ using ftcuda::LaunchState;
 
 static_assert(std::is_trivially_copyable<LaunchState>::value, "a launch must be copyable with the Primitive");
 
+// The TF32 family behind a prepared one (and, where an operand's magnitudes spread too far, in its place), or -1.
+int fallbackOf(int kernel) {
+    switch (kernel) {
+        case FTCUDA_GEMM_FP16X3: return FTCUDA_GEMM_TF32X3;
+        case FTCUDA_GEMM_FP16X3_SPLITK: return FTCUDA_GEMM_TF32X3_SPLITK;
+        default: return -1;
+    }
+}
+
 bool stagesOperands(int kernel) {
     return kernel == FTCUDA_GEMM_TF32X3 || kernel == FTCUDA_GEMM_TF32X3_SPLITK || kernel == FTCUDA_GEMM_TF32X3_ROWS;
 }
@@ -21,6 +30,10 @@ const char* supportsAsGiven(int kernel, const FtcudaGemmDesc& desc);
 // The tensor-core families take operands TMA cannot describe through a copy in the workspace: their
 // own rules are asked about the problem with those operands replaced by the copies' description.
 const char* supports(int kernel, const FtcudaGemmDesc& desc) {
+    if (const int fallback = fallbackOf(kernel); fallback >= 0) {
+        const char* reason = ftcuda::supportsPrepared(desc);
+        return reason != nullptr ? reason : supports(fallback, desc);
+    }
     if (!stagesOperands(kernel)) { return supportsAsGiven(kernel, desc); }
     LaunchState probe{};
     probe.desc = desc;
@@ -42,6 +55,19 @@ const char* supportsAsGiven(int kernel, const FtcudaGemmDesc& desc) {
 
 }  // namespace
 
+// Copies the operands TMA cannot fetch into the head of the workspace, points the launch's descriptors at
+// them, and hands the rest of the workspace to the kernel family.
+cudaError_t ftcuda::launchTensorStaged(LaunchState& local, void* workspace, cudaStream_t stream, char* message,
+                                       std::size_t capacity) {
+    void* rest = workspace;
+    if (local.staged != 0) {
+        const cudaError_t error = runStaging(local, workspace, stream, message, capacity);
+        if (error != cudaSuccess) { return error; }
+        rest = static_cast<unsigned char*>(workspace) + local.stage_bytes;
+    }
+    return local.kernel == FTCUDA_GEMM_TF32X3_ROWS ? launchTensorRows(local, stream) : launchTensor(local, rest, stream);
+}
+
 extern "C" int ftcuda_gemm_supports(int kernel, const FtcudaGemmDesc* desc, char* message, size_t message_capacity) {
     if (desc == nullptr) { return ftcuda::fail(message, message_capacity, 1, "null descriptor"); }
     const char* reason = supports(kernel, *desc);
@@ -55,9 +81,12 @@ extern "C" int ftcuda_gemm_configure(int kernel, const FtcudaGemmDesc* desc, Ftc
     const char* reason = supports(kernel, *desc);
     if (reason != nullptr) { return ftcuda::fail(message, message_capacity, 1, "%s", reason); }
     std::memset(launch, 0, sizeof *launch);
-    LaunchState& state = *reinterpret_cast<LaunchState*>(launch);
-    state.desc         = *desc;
-    state.kernel       = kernel;
+    LaunchState& state  = *reinterpret_cast<LaunchState*>(launch);
+    const int requested = kernel;
+    const bool prepared = fallbackOf(kernel) >= 0;
+    if (prepared) { kernel = fallbackOf(kernel); }
+    state.desc   = *desc;
+    state.kernel = kernel;
     if (stagesOperands(kernel)) {
         // state.desc now describes the copies; the family configures itself for them.
         if (const char* staging = ftcuda::planStaging(kernel, *desc, state)) { return ftcuda::fail(message, message_capacity, 1, "%s", staging); }
@@ -75,6 +104,11 @@ extern "C" int ftcuda_gemm_configure(int kernel, const FtcudaGemmDesc* desc, Ftc
         // The copies take the head of the workspace (plus room to align them), the family's own needs follow.
         state.stage_bytes += 256;
         state.workspace_bytes += state.stage_bytes;
+    }
+    if (status == 0 && prepared) {
+        status                         = ftcuda::configurePrepared(state, *desc, message, message_capacity);
+        state.prepared.fallback_kernel = kernel;
+        state.kernel                   = requested;
     }
     return status;
 }
@@ -98,24 +132,18 @@ extern "C" int ftcuda_gemm_launch(const FtcudaGemmLaunch* launch, void* workspac
     }
     const cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
     cudaError_t error              = cudaSuccess;
-    if (state.staged != 0) {
-        // Copy the operands TMA cannot fetch into the head of the workspace, point a copy of the launch's
-        // descriptors at them, and hand the rest of the workspace to the kernel family.
-        LaunchState local = state;
+    if (state.staged != 0 || state.prepared.fallback_kernel != 0) {
         if (message != nullptr && message_capacity != 0) { message[0] = '\0'; }
-        error = ftcuda::runStaging(local, workspace, cuda_stream, message, message_capacity);
+        if (state.prepared.fallback_kernel != 0) {
+            error = ftcuda::launchPrepared(state, workspace, cuda_stream, message, message_capacity);
+        } else {
+            LaunchState local = state;
+            error             = ftcuda::launchTensorStaged(local, workspace, cuda_stream, message, message_capacity);
+        }
         if (error != cudaSuccess) {
             if (message != nullptr && message_capacity != 0 && message[0] != '\0') { return 1; }
             return ftcuda::fail(message, message_capacity, 1, "%s", cudaGetErrorString(error));
         }
-        void* const rest = static_cast<unsigned char*>(workspace) + local.stage_bytes;
-        local.workspace_bytes -= local.stage_bytes;
-        if (local.kernel == FTCUDA_GEMM_TF32X3_ROWS) {
-            error = ftcuda::launchTensorRows(local, cuda_stream);
-        } else {
-            error = ftcuda::launchTensor(local, rest, cuda_stream);
-        }
-        if (error != cudaSuccess) { return ftcuda::fail(message, message_capacity, 1, "%s", cudaGetErrorString(error)); }
         return 0;
     }
     switch (state.kernel) {

@@ -177,6 +177,28 @@ bool encodeTensorMap2d(CUtensorMap* map, const void* base, std::uint64_t inner, 
     return true;
 }
 
+bool encodeSplitMap(CUtensorMap* map, const void* base, std::uint64_t rows, std::uint64_t blocks, std::uint32_t box_rows,
+                    char* message, std::size_t capacity) {
+    const PFN_cuTensorMapEncodeTiled_v12000 encode = tensorMapEncoder();
+    if (encode == nullptr) {
+        fail(message, capacity, 1, "the CUDA driver does not provide cuTensorMapEncodeTiled");
+        return false;
+    }
+    // [64 of a half-block][row][half-block]: one copy brings the high and the low tile, one after the other.
+    const cuuint64_t dims[3]     = {64, rows, 2 * blocks};
+    const cuuint64_t strides[2]  = {blocks * 256, 128};
+    const cuuint32_t box[3]      = {64, box_rows, 2};
+    const cuuint32_t elements[3] = {1, 1, 1};
+    const CUresult result = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, elements,
+                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (result != CUDA_SUCCESS) {
+        fail(message, capacity, 1, "cuTensorMapEncodeTiled failed with CUresult %d", static_cast<int>(result));
+        return false;
+    }
+    return true;
+}
+
 void countLaunches(std::uint64_t launches) { g_launches.fetch_add(launches, std::memory_order_relaxed); }
 
 }  // namespace ftcuda

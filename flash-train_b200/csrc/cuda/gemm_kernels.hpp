@@ -36,6 +36,20 @@ struct StagedOperand {
     std::uint64_t offset;                  // byte offset of the copy in the workspace, a multiple of 256
 };
 
+// The prepared form of a tensor-core launch (gemm_fp16x3.cu): its own geometry and the layout of the
+// workspace. The rest of the LaunchState is the TF32 launch that takes over when the operands' magnitudes
+// spread too far for it.
+struct PreparedState {
+    alignas(64) CUtensorMap map_a;
+    alignas(64) CUtensorMap map_b;
+    FtcudaGemmDesc desc;           // as the caller gave it (LaunchState::desc may describe staged copies)
+    std::int32_t fallback_kernel;  // 0 is never a fallback: nonzero marks a prepared launch
+    std::uint32_t tile_n, splits, blocks_per_split, chunk_blocks;
+    std::uint32_t grid;
+    std::uint64_t cleared_bytes;                  // head of the workspace cleared before the launch
+    std::uint64_t max_at[2], few_at[2], inverse_at[2], split_at[2], partials_at;
+};
+
 // What ftcuda_gemm_configure stores inside an FtcudaGemmLaunch.
 struct LaunchState {
     alignas(64) CUtensorMap map_a;
@@ -61,6 +75,10 @@ struct LaunchState {
     std::uint32_t staged;          // bit 0: A is staged, bit 1: B
     StagedOperand stage[2];
     std::uint64_t stage_bytes;     // bytes at the head of the workspace taken by the copies
+    // Set only in the copy of a launch that serves as a prepared launch's fallback: its kernels run when *run_if
+    // is nonzero and leave at once otherwise.
+    const std::uint32_t* run_if;
+    PreparedState prepared;
 };
 static_assert(sizeof(LaunchState) <= sizeof(FtcudaGemmLaunch), "launch blob too small");
 static_assert(alignof(FtcudaGemmLaunch) >= 64, "launch blob must be 64-byte aligned");
@@ -95,6 +113,11 @@ bool encodeTensorMap2d(CUtensorMap* map, const void* base, std::uint64_t inner, 
                        std::uint64_t row_pitch_bytes, std::uint32_t box_inner, std::uint32_t box_outer,
                        int swizzle, char* message, std::size_t capacity);
 void countLaunches(std::uint64_t launches);
+
+// 3-D FP16 map over a split operand: `rows` rows of `blocks` 64-element blocks, 128-byte swizzle, box 64 x box_rows x 2.
+bool encodeSplitMap(CUtensorMap* map, const void* base, std::uint64_t rows, std::uint64_t blocks, std::uint32_t box_rows,
+                    char* message, std::size_t capacity);
+bool replaceMapAddress(CUtensorMap* map, void* base);
 
 // True when `base`/strides describe a matrix TMA can fetch with `contiguous`
 // as the unit-stride dimension: unit stride there, 16-byte aligned base,
@@ -173,9 +196,20 @@ int configureTensorGrouped(GroupedLaunchState& state, const FtcudaGemmDesc* grou
                            std::size_t capacity);
 cudaError_t launchTensorGrouped(const GroupedLaunchState& state, void* workspace, cudaStream_t stream);
 
-// D = alpha * sum_s partial[s] + beta * C over `splits` dense m x n partials.
+// D = alpha * sum_s partial[s] + beta * C over `splits` dense m x n partials. With `decision`, only if
+// (*decision != 0) == run_when.
 cudaError_t launchSplitKReduce(const FtcudaGemmDesc& desc, const float* partials, std::uint32_t splits,
-                               cudaStream_t stream);
+                               cudaStream_t stream, const std::uint32_t* decision = nullptr, bool run_when = true);
+
+// ---- the prepared form (gemm_fp16x3.cu) ----
+const char* supportsPrepared(const FtcudaGemmDesc& desc);
+// `state` is the configured fallback; adds the prepared part and raises workspace_bytes to what both need.
+int configurePrepared(LaunchState& state, const FtcudaGemmDesc& desc, char* message, std::size_t capacity);
+// Enqueues the split, the FP16 kernel and (after it, guarded) the fallback.
+cudaError_t launchPrepared(const LaunchState& state, void* workspace, cudaStream_t stream, char* message, std::size_t capacity);
+// The rest of ftcuda_gemm_launch for the tensor-core families: staging, then the kernel.
+cudaError_t launchTensorStaged(LaunchState& local, void* workspace, cudaStream_t stream, char* message,
+                               std::size_t capacity);
 
 }  // namespace ftcuda
 

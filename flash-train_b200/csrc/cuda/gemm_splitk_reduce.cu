@@ -23,12 +23,15 @@ struct ReduceParams {
     std::uint32_t splits;
     float alpha, beta;
     bool vectorised;
+    bool run_when;
+    const std::uint32_t* decision;
 };
 
 __global__ void __launch_bounds__(256) splitKReduce(const ReduceParams p) {
     // Launched with programmatic stream serialization: the CTAs may be resident before the kernel
     // that writes the partial sums has completed, and wait here for it.
     gridDependencyWait();
+    if (p.decision != nullptr && (*p.decision != 0) != p.run_when) { return; }
     const std::uint64_t slab   = p.m * p.n;
     const std::uint64_t stride = static_cast<std::uint64_t>(gridDim.x) * blockDim.x;
     std::uint64_t index        = static_cast<std::uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -101,8 +104,10 @@ bool denseAligned(const float* base, std::int64_t row_stride, std::int64_t col_s
 }  // namespace
 
 cudaError_t launchSplitKReduce(const FtcudaGemmDesc& desc, const float* partials, std::uint32_t splits,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, const std::uint32_t* decision, bool run_when) {
     ReduceParams p{};
+    p.decision     = decision;
+    p.run_when     = run_when;
     p.partials     = partials;
     p.c            = desc.c;
     p.d            = desc.d;

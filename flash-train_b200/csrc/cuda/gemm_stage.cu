@@ -27,6 +27,7 @@ struct RepackParams {
     std::uint64_t rows, cols;
     float* copy;
     std::uint64_t pitch;
+    const std::uint32_t* run_if;
 };
 
 // 32 x 32 elements per CTA. When the source runs fastest along its rows index (a transposed view)
@@ -34,6 +35,7 @@ struct RepackParams {
 // consecutive addresses; otherwise it is a straight strided copy.
 __global__ void __launch_bounds__(256) repackMatrix(const RepackParams p) {
     __shared__ float tile[32][33];
+    if (p.run_if != nullptr && *p.run_if == 0) { return; }
     const std::uint64_t row0 = static_cast<std::uint64_t>(blockIdx.x) * 32;
     const std::uint64_t col0 = static_cast<std::uint64_t>(blockIdx.y) * 32;
     const int tx             = threadIdx.x & 31;
@@ -144,6 +146,11 @@ const char* planStaging(int kernel, const FtcudaGemmDesc& desc, LaunchState& sta
     return nullptr;
 }
 
+bool replaceMapAddress(CUtensorMap* map, void* base) {
+    const PFN_cuTensorMapReplaceAddress_v12000 replace = addressReplacer();
+    return replace != nullptr && replace(map, base) == CUDA_SUCCESS;
+}
+
 cudaError_t runStaging(LaunchState& local, void* workspace, cudaStream_t stream, char* message, std::size_t capacity) {
     const PFN_cuTensorMapReplaceAddress_v12000 replace = addressReplacer();
     if (replace == nullptr) {
@@ -163,6 +170,7 @@ cudaError_t runStaging(LaunchState& local, void* workspace, cudaStream_t stream,
         p.cols       = staged.cols;
         p.copy       = reinterpret_cast<float*>(base + staged.offset);
         p.pitch      = staged.pitch;
+        p.run_if     = local.run_if;
         const dim3 grid(static_cast<unsigned>(ceilDiv(staged.rows, 32)), static_cast<unsigned>(ceilDiv(staged.cols, 32)), 1);
         repackMatrix<<<grid, 256, 0, stream>>>(p);
         const cudaError_t error = cudaGetLastError();

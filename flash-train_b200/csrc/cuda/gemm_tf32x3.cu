@@ -144,6 +144,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 tensorGemm3xTf32(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const TensorParams p, const std::uint32_t num_items) {
     extern __shared__ unsigned char smem_raw[];
+    if (p.run_if != nullptr) {
+        gridDependencyWait();  // the cluster form may start early
+        if (*p.run_if == 0) { return; }
+    }
     const std::uint32_t align_offset = (1024 - (smemAddress(smem_raw) & 1023)) & 1023;
     unsigned char* smem              = smem_raw + align_offset;
     Barriers* bars                   = reinterpret_cast<Barriers*>(smem + kBarrierOffset);
@@ -781,6 +785,7 @@ TensorParams makeTensorParams(const LaunchState& state) {
     p.alpha          = desc.alpha;
     p.beta           = desc.beta;
     p.status         = state.device_status;
+    p.run_if         = state.run_if;
     return p;
 }
 
@@ -819,7 +824,7 @@ cudaError_t launchTensor(const LaunchState& state, void* workspace, cudaStream_t
     error = cudaGetLastError();
     std::uint64_t launches = 1;
     if (error == cudaSuccess && state.splits > 1) {
-        error = launchSplitKReduce(desc, static_cast<const float*>(workspace), state.splits, stream);
+        error = launchSplitKReduce(desc, static_cast<const float*>(workspace), state.splits, stream, state.run_if);
         ++launches;
     }
     countLaunches(launches);

@@ -365,6 +365,70 @@ __device__ __forceinline__ void tmemStore16NoWait(std::uint32_t address, const f
 
 __device__ __forceinline__ void tmemStoreWait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// ---------------------------------------------------------------- CTA pairs (tcgen05 cta_group::2)
+// Two CTAs of a cluster of two, on neighbouring SMs, share one MMA: 256 rows of D, 128 in each CTA's tensor
+// memory, A's rows and half of B's rows from each CTA's shared memory at the same offsets.
+
+// Address of this CTA's shared-memory object in the CTA of rank `rank`, for .shared::cluster accesses.
+__device__ __forceinline__ std::uint32_t mapToRank(const void* pointer, std::uint32_t rank) {
+    std::uint32_t mapped;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(mapped) : "r"(smemAddress(pointer)), "r"(rank));
+    return mapped;
+}
+
+// Arrives on a barrier of any CTA of the cluster (an address from mapToRank).
+__device__ __forceinline__ void mbarrierArriveCluster(std::uint32_t barrier) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(barrier) : "memory");
+}
+
+// Whole-warp calls, made by one warp of each CTA of the pair.
+__device__ __forceinline__ void tmemAllocatePair(std::uint32_t* result_in_smem, std::uint32_t columns) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddress(result_in_smem)),
+                 "r"(columns)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmemFreePair(std::uint32_t base, std::uint32_t columns) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns) : "memory");
+}
+
+// 3-D tiled load into this CTA's shared memory; the bytes count on `barrier` (an address from mapToRank), which may
+// be the pair's other CTA's. No multicast: each CTA fetches its own tile.
+__device__ __forceinline__ void tmaLoad3dPair(void* smem_destination, const void* tensor_map, std::uint32_t barrier,
+                                              std::int32_t x, std::int32_t y, std::int32_t z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smemAddress(smem_destination)),
+        "l"(reinterpret_cast<std::uint64_t>(tensor_map)), "r"(barrier), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+
+// Instruction descriptor for kind::f16 with FP16 operands (format 0), FP32 accumulation, both operands K-major.
+__host__ __device__ constexpr std::uint32_t umaInstructionF16(std::uint32_t m, std::uint32_t n) {
+    return (1u << 4) | ((n >> 3) << 17) | ((m >> 4) << 24);
+}
+
+// D[tmem] (+)= A[smem] * B[smem] over the pair; issued by ONE thread of its first CTA.
+__device__ __forceinline__ void umaF16Pair(std::uint32_t d_tmem, std::uint64_t a_descriptor, std::uint64_t b_descriptor,
+                                           std::uint32_t instruction, std::uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+        "}" ::"r"(d_tmem),
+        "l"(a_descriptor), "l"(b_descriptor), "r"(instruction), "r"(accumulate)
+        : "memory");
+}
+
+// Arrives once on `barrier` of BOTH CTAs when every MMA this thread issued so far has finished.
+__device__ __forceinline__ void umaCommitPair(std::uint64_t* barrier) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                     smemAddress(barrier)),
+                 "h"(static_cast<std::uint16_t>(3))
+                 : "memory");
+}
+
 }  // namespace ftcuda
 
 #endif

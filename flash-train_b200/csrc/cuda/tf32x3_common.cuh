@@ -50,6 +50,8 @@ struct TensorParams {
     // Grouped launches: the per-group table and, per work item, the index of its group.
     const GroupEntry* groups;
     const std::uint32_t* item_group;
+    // The fallback of a prepared launch: the kernel leaves at once unless *run_if is nonzero.
+    const std::uint32_t* run_if;
 };
 
 // Grouped launches (one persistent launch over the output tiles of many independent GEMMs): one

@@ -10,6 +10,14 @@ std::uint64_t ceilDiv(std::uint64_t x, std::uint64_t y) { return (x + y - 1) / y
 
 }  // namespace
 
+// The split reads A and B twice and writes them once, about 35 us of launches and memory passes before the first
+// MMA; the multiplication then takes half the time. Measured (TF32 form / prepared form, microseconds):
+// 2048^3 114 / 98, 4096 x 4096 x 2048 362 / 270, 4096^3 688 / 471, 16384 x 4096 x 14336 8810 / 4520; but
+// 1024^3 25 / 50, 2048 x 8192 x 1024 172 / 194, 1024 x 8192 x 2048 168 / 194.
+bool preparedFormPays(const GemmShape& shape) noexcept {
+    return shape.m >= 2048 && shape.n >= 2048 && shape.k >= 2048;
+}
+
 // Regime map on B200 (148 SMs; the count is queried, not assumed). The
 // thresholds come from timing every kernel family on a grid of shapes
 // (bench.py --workload finder_sweep) and keeping the Finder's first choice

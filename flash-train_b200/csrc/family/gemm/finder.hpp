@@ -21,6 +21,10 @@ struct B200Heuristic final {
     static std::vector<std::string> findCandidates(const GemmProblem& problem, const Constraints& constraints);
 };
 
+// Whether splitting the operands first (the prepared form of the tensor-core families) is
+// faster than splitting them on the way, for a caller that gives the workspace.
+bool preparedFormPays(const GemmShape& shape) noexcept;
+
 // Kept so that FTRAIN_DISABLED_FINDERS=B200Heuristic reproduces the
 // reference's behaviour: no opinion, registration order decides.
 struct RegistrationOrderFinder final {

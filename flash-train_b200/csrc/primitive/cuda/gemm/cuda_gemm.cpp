@@ -2,6 +2,8 @@
 
 #include <cstdint>
 
+#include "family/gemm/finder.hpp"
+
 namespace ftrain {
 namespace {
 
@@ -12,6 +14,15 @@ bool floatAligned(const void* address) noexcept {
 constexpr GemmPort kAllPorts[]    = {GemmPort::kA, GemmPort::kB,     GemmPort::kC,
                                      GemmPort::kD, GemmPort::kAlpha, GemmPort::kBeta};
 constexpr GemmPort kMatrixPorts[] = {GemmPort::kA, GemmPort::kB, GemmPort::kC, GemmPort::kD};
+
+// The prepared form of a kernel family, or -1.
+int preparedForm(int kernel) noexcept {
+    switch (kernel) {
+        case FTCUDA_GEMM_TF32X3: return FTCUDA_GEMM_FP16X3;
+        case FTCUDA_GEMM_TF32X3_SPLITK: return FTCUDA_GEMM_FP16X3_SPLITK;
+        default: return -1;
+    }
+}
 
 }  // namespace
 
@@ -101,6 +112,7 @@ Result CudaGemm::isApplicable(const GemmProblem& problem, const Constraints& con
 void CudaGemm::configure(const GemmProblem& problem) {
     empty_           = problem.hasEmptyOutput();
     workspace_bytes_ = 0;
+    prepared_bytes_  = 0;
     if (empty_) { return; }
     const FtcudaGemmDesc desc = makeCudaGemmDesc(problem, getCurrentDeviceId(), true);
     char reason[256];
@@ -109,13 +121,28 @@ void CudaGemm::configure(const GemmProblem& problem) {
         throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "%s: configuring the launch failed: %s", getName(), reason);
     }
     workspace_bytes_ = ftcuda_gemm_workspace_bytes(&launch_);
+    const int prepared = preparedForm(kernel_);
+    if (prepared >= 0 && preparedFormPays(problem.getShape()) && ftcuda_gemm_supports(prepared, &desc, reason, sizeof reason) == 0) {
+        if (ftcuda_gemm_configure(prepared, &desc, &prepared_, reason, sizeof reason) != 0) {
+            throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "%s: configuring the launch failed: %s", getName(), reason);
+        }
+        prepared_bytes_ = ftcuda_gemm_workspace_bytes(&prepared_);
+    }
+}
+
+std::unique_ptr<PrimitiveBase> CudaGemm::cloneForMinimumWorkspace() const {
+    if (prepared_bytes_ == 0) { return nullptr; }
+    auto lean             = std::make_unique<CudaGemm>(*this);
+    lean->prepared_bytes_ = 0;
+    return lean;
 }
 
 void CudaGemm::executeImpl(const Resources& resources) {
     if (empty_) { return; }
     char reason[256];
     reason[0] = '\0';
-    if (ftcuda_gemm_launch(&launch_, resources.getWorkspace(), resources.getWorkspaceBytes(), resources.getStream(),
+    const bool prepared = prepared_bytes_ != 0 && resources.getWorkspace() != nullptr && resources.getWorkspaceBytes() >= prepared_bytes_;
+    if (ftcuda_gemm_launch(prepared ? &prepared_ : &launch_, resources.getWorkspace(), resources.getWorkspaceBytes(), resources.getStream(),
                            reason, sizeof reason) != 0) {
         throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "FP32 GEMM kernel launch failed: %s", reason);
     }

@@ -38,7 +38,11 @@ class CudaGemm final : public Primitive<GemmProblem> {
     const char* getName() const noexcept override { return cudaGemmName(kernel_); }
     std::unique_ptr<PrimitiveBase> clone() const override { return std::make_unique<CudaGemm>(*this); }
     Result isApplicable(const GemmProblem& problem, const Constraints& constraints) const override;
-    std::uint64_t getRequiredWorkspaceBytes() const noexcept override { return workspace_bytes_; }
+    std::uint64_t getRequiredWorkspaceBytes() const noexcept override {
+        return prepared_bytes_ != 0 ? prepared_bytes_ : workspace_bytes_;
+    }
+    std::uint64_t getMinimumWorkspaceBytes() const noexcept override { return workspace_bytes_; }
+    std::unique_ptr<PrimitiveBase> cloneForMinimumWorkspace() const override;
     // Binds to the calling thread's current device.
     void configure(const GemmProblem& problem) override;
 
@@ -49,6 +53,10 @@ class CudaGemm final : public Primitive<GemmProblem> {
     bool empty_{true};  // nothing to launch (m * n == 0, or not configured)
     std::uint64_t workspace_bytes_{0};
     FtcudaGemmLaunch launch_{};
+    // The family's prepared form (FTCUDA_GEMM_FP16X3...), where it exists and pays: used whenever
+    // the caller's workspace holds prepared_bytes_ (0: there is none).
+    std::uint64_t prepared_bytes_{0};
+    FtcudaGemmLaunch prepared_{};
 };
 
 }  // namespace ftrain

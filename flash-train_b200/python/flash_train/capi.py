@@ -455,6 +455,8 @@ KERNEL_TF32X3_SPLITK = 2
 KERNEL_SKINNY = 3
 KERNEL_SIMT_SPLITK = 4
 KERNEL_TF32X3_ROWS = 5
+KERNEL_FP16X3 = 6  # the prepared forms of KERNEL_TF32X3 and KERNEL_TF32X3_SPLITK
+KERNEL_FP16X3_SPLITK = 7
 KERNEL_NAMES = {
     KERNEL_SIMT: "Fp32Gemm",
     KERNEL_TF32X3: "Fp32Gemm3xTf32",

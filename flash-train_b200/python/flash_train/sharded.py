@@ -77,10 +77,12 @@ class _LibraryGemm:
                 capi.tensor_operand(c) if c is not None else capi.null_operand(rows, cols),
                 capi.tensor_operand(d), alpha, beta)
             size = plan.workspace_bytes(0)
-            workspace = torch.empty(max(size, 1), dtype=torch.uint8, device=a.device)
-            entry = (plan, workspace, size)
+            entry = (plan, size)
             self._plans[key] = entry
-        plan, workspace, size = entry
+        plan, size = entry
+        # From the caching allocator on every call: the block belongs to the current stream, and the
+        # Plans kept here do not each hold one.
+        workspace = torch.empty(max(size, 1), dtype=torch.uint8, device=a.device)
         plan.execute(0, workspace.data_ptr() if size else 0, size, torch.cuda.current_stream(a.device).cuda_stream)
 
 

@@ -148,6 +148,31 @@ bool planReuseDisabled() {
     return disabled;
 }
 
+// Runs the Plan's first primitive whose workspace torch's allocator can give: the best form of a tensor-core
+// family takes as much memory as A and B, and the primitives behind it do with less.
+FTrainStatus executePlan(FTrainPlan plan, std::uint64_t first_bytes, const at::TensorOptions& options, FTrainStream stream) {
+    std::uint64_t bytes = first_bytes;
+    for (std::uint64_t index = 0;; ++index) {
+        if (index != 0) {
+            const FTrainStatus status = ftrainPlanGetPrimitiveRequiredWorkspaceBytes(plan, index, &bytes);
+            if (status != FTRAIN_STATUS_SUCCESS) { return status; }
+        }
+        at::Tensor workspace;
+        if (bytes != 0) {
+            try {
+                workspace = torch::empty({static_cast<std::int64_t>(bytes)}, options.dtype(at::kByte));
+            } catch (const c10::OutOfMemoryError&) {
+                std::uint64_t count = 0;
+                if (ftrainPlanGetNumPrimitives(plan, &count) != FTRAIN_STATUS_SUCCESS || index + 1 >= count) { throw; }
+                continue;
+            }
+        }
+        // The caching allocator keeps the block reserved for this stream until
+        // the enqueued work is done, so `workspace` may go out of scope.
+        return ftrainPlanExecutePrimitive(plan, index, bytes != 0 ? workspace.data_ptr() : nullptr, bytes, stream);
+    }
+}
+
 at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const std::optional<at::Tensor>& c, double alpha,
                 double beta) {
     checkMatrix(a, "a");
@@ -187,12 +212,7 @@ at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const std::optional<at
     key.device = a.device().index();
     if (reuse) {
         if (RecentPlans::Entry* known = recent.find(key)) {
-            at::Tensor scratch;
-            if (known->workspace_bytes != 0) {
-                scratch = torch::empty({static_cast<std::int64_t>(known->workspace_bytes)}, a.options().dtype(at::kByte));
-            }
-            const FTrainStatus again = ftrainPlanExecutePrimitive(
-                known->plan, 0, known->workspace_bytes != 0 ? scratch.data_ptr() : nullptr, known->workspace_bytes, stream);
+            const FTrainStatus again = executePlan(known->plan, known->workspace_bytes, a.options(), stream);
             TORCH_CHECK(again == FTRAIN_STATUS_SUCCESS, "flash_train gemm failed with status ", static_cast<unsigned>(again), ": ",
                         ftrainGetLastMessage());
             return d;
@@ -221,16 +241,7 @@ at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const std::optional<at
     if (status == FTRAIN_STATUS_SUCCESS) { status = ftrainPlanCreate(&plan, args); }
     std::uint64_t workspace_bytes = 0;
     if (status == FTRAIN_STATUS_SUCCESS) { status = ftrainPlanGetPrimitiveRequiredWorkspaceBytes(plan, 0, &workspace_bytes); }
-    at::Tensor workspace;
-    if (status == FTRAIN_STATUS_SUCCESS) {
-        if (workspace_bytes != 0) {
-            workspace = torch::empty({static_cast<std::int64_t>(workspace_bytes)}, a.options().dtype(at::kByte));
-        }
-        // The caching allocator keeps the block reserved for this stream until
-        // the enqueued work is done, so `workspace` may go out of scope below.
-        status = ftrainPlanExecutePrimitive(plan, 0, workspace_bytes != 0 ? workspace.data_ptr() : nullptr,
-                                            workspace_bytes, stream);
-    }
+    if (status == FTRAIN_STATUS_SUCCESS) { status = executePlan(plan, workspace_bytes, a.options(), stream); }
     const std::string failure = status == FTRAIN_STATUS_SUCCESS ? std::string() : std::string(ftrainGetLastMessage());
     if (status == FTRAIN_STATUS_SUCCESS && reuse) {
         recent.insert(key, plan, workspace_bytes);  // kept for the next call with these tensors

@@ -50,7 +50,13 @@ enum {
     /* 3xTF32 for few rows of A (m <= 64): B fills the tensor core's 128-row
      * dimension (D^T = B^T A^T), K split over a thread-block cluster. No workspace. */
     FTCUDA_GEMM_TF32X3_ROWS = 5,
-    FTCUDA_GEMM_KERNEL_COUNT = 6,
+    /* The prepared forms of FTCUDA_GEMM_TF32X3 and FTCUDA_GEMM_TF32X3_SPLITK: the launch splits the operands into
+     * scaled FP16 pairs in the workspace (as many bytes as A and B) and multiplies those at twice the TF32 rate,
+     * with no larger error. Operands whose magnitudes spread too far within a row of A or a column of B
+     * (or are not finite) go through the TF32 family instead; the GPU decides, in the launch. */
+    FTCUDA_GEMM_FP16X3 = 6,
+    FTCUDA_GEMM_FP16X3_SPLITK = 7,
+    FTCUDA_GEMM_KERNEL_COUNT = 8,
 };
 
 /* One GEMM D = alpha * A * B + beta * C in terms of raw memory. Strides are in

@@ -1,0 +1,128 @@
+"""The prepared form of the 3xTF32 families (operands split into scaled FP16 pairs first): every edge of its tiles and
+splits against float64, and the operands it has to leave to the TF32 kernel."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ERROR_FLOOR = 2.0 ** -24
+
+
+@pytest.fixture(scope="module")
+def gpu(capi):
+    import gpu_support
+
+    return gpu_support
+
+
+def run(capi, gpu, kernel, a, b, c, alpha, beta, out=None):
+    m, n = a.shape[0], b.shape[1]
+    d = out if out is not None else torch.full((m, n), float("nan"), device="cuda")
+    desc = capi.make_desc(gpu.operand(a), gpu.operand(b), gpu.operand(c) if c is not None else capi.null_operand(m, n),
+                          gpu.operand(d), alpha, beta, 0)
+    assert capi.platform_supports(kernel, desc) is None
+    launch = capi.PlatformGemm(kernel, desc)
+    workspace = torch.full((launch.workspace_bytes + 4,), 255, dtype=torch.uint8, device="cuda")
+    launch.run(workspace.data_ptr() + 4, launch.workspace_bytes, gpu.current_stream())  # any alignment must do
+    torch.cuda.synchronize()
+    return d
+
+
+def check(oracle, d, a, b, c, alpha, beta, what):
+    exact = alpha * (a.double() @ b.double()) + (beta * c.double() if c is not None else 0.0)
+    ours = oracle.scaled_error(d, exact, a * abs(alpha), b, c, beta)
+    plain = oracle.scaled_error(oracle.torch_reference(a, b, c, alpha, beta), exact, a * abs(alpha), b, c, beta)
+    assert torch.isfinite(d).all() and ours <= 2.0 * max(plain, ERROR_FLOOR), f"{what}: {ours:.3e} against {plain:.3e}"
+
+
+@pytest.mark.parametrize("m,k,n", [
+    (1, 256, 1),          # the smallest it takes: one row, one column
+    (255, 257, 63),       # just under a tile, one K value over a block
+    (257, 448, 257),      # one row and one column over a tile
+    (300, 1003, 501),     # nothing aligned
+    (1500, 512, 700),     # several tiles, a whole number of K blocks
+    (129, 5000, 130),     # K slices
+    (640, 2048, 4740),    # several waves of tiles on few rows
+])
+def test_shapes_and_layouts(capi, gpu, oracle, m, k, n):
+    torch.manual_seed(m + k + n)
+    a, b, c = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda"), torch.randn(m, n, device="cuda")
+    a_t, b_t = a.t().contiguous().t(), b.t().contiguous().t()
+    a_odd = torch.empty(m, k + 3, device="cuda")[:, 1:k + 1].copy_(a)        # unaligned rows
+    b_wide = torch.empty(k, 2 * n, device="cuda")[:, ::2].copy_(b)          # no unit stride at all
+    d_odd = torch.full((n, m + 1), float("nan"), device="cuda")[:, :m].t()  # D written through strides
+    for kernel in (capi.KERNEL_FP16X3, capi.KERNEL_FP16X3_SPLITK):
+        if kernel == capi.KERNEL_FP16X3_SPLITK and k < 512:
+            continue
+        check(oracle, run(capi, gpu, kernel, a, b, None, 1.0, 0.0), a, b, None, 1.0, 0.0, "plain")
+        check(oracle, run(capi, gpu, kernel, a_t, b_t, c, 1.5, -0.25), a, b, c, 1.5, -0.25, "both transposed, C")
+        check(oracle, run(capi, gpu, kernel, a_odd, b_wide, c, -1.0, 0.5, out=d_odd), a, b, c, -1.0, 0.5, "strided")
+        in_place = c.clone()
+        run(capi, gpu, kernel, a, b_t, in_place, 1.0, 2.0, out=in_place)
+        check(oracle, in_place, a, b, c, 1.0, 2.0, "in place")
+        again = run(capi, gpu, kernel, a, b, None, 1.0, 0.0)
+        assert torch.equal(again, run(capi, gpu, kernel, a, b, None, 1.0, 0.0)), "results repeat bit for bit"
+
+
+def test_scales_of_rows_and_columns(capi, gpu, oracle):
+    """Rows of A and columns of B of very different size, and rows without a single nonzero."""
+    torch.manual_seed(1)
+    m, k, n = 300, 700, 270
+    a = torch.randn(m, k, device="cuda") * torch.exp2(torch.randint(-40, 40, (m, 1), device="cuda").float())
+    b = torch.randn(k, n, device="cuda") * torch.exp2(torch.randint(-40, 40, (1, n), device="cuda").float())
+    a[7], a[:, 3], b[:, 11] = 0.0, 0.0, 0.0
+    d = run(capi, gpu, capi.KERNEL_FP16X3, a, b, None, 1.0, 0.0)
+    exact = a.double() @ b.double()
+    bound = (a.double().norm(dim=1, keepdim=True) * b.double().norm(dim=0, keepdim=True)) * 2.0 ** -22
+    assert ((d.double() - exact).abs() <= bound).all() and (d[7] == 0).all() and (d[:, 11] == 0).all()
+
+
+@pytest.mark.parametrize("kind", ["depth", "pair", "sparse", "large", "tiny", "inf", "nan"])
+def test_operands_left_to_the_tf32_kernel(capi, gpu, kind):
+    """Magnitudes that spread too far for scaled FP16 pairs (or are not finite): the result is bit for bit that of
+    the TF32 family -- also where C is D, which nothing may have written before the decision."""
+    torch.manual_seed(2)
+    m, k, n = 300, 1000, 270
+    a, b = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda")
+    if kind == "depth":  # A and B scaled against each other along K
+        scale = torch.exp2(torch.randint(-30, 30, (k,), device="cuda").float())
+        a, b = a * scale, b / scale[:, None]
+    elif kind == "pair":  # one row of A and one column of B that meet in a pair of far smaller elements
+        a[5], b[:, 9] = 0.0, 0.0
+        a[5, 0], a[5, 1], b[0, 9], b[1, 9] = 2.0 ** 40, 1.0, 2.0 ** -40, 1.0
+    elif kind == "sparse":  # hardly any elements of full size to hide the small ones behind
+        a[:, 10:] *= 2.0 ** -30
+        b[:, 10:] *= 2.0 ** -30
+    elif kind == "large":
+        a[3, 4] = 2.0 ** 110
+    elif kind == "tiny":
+        b[:, 5] *= 2.0 ** -120
+    elif kind == "inf":
+        a[3, 4] = float("inf")
+    else:
+        b[3, 4] = float("nan")
+    c = torch.randn(m, n, device="cuda")
+    for prepared, plain in ((capi.KERNEL_FP16X3, capi.KERNEL_TF32X3), (capi.KERNEL_FP16X3_SPLITK, capi.KERNEL_TF32X3_SPLITK)):
+        one, other = c.clone(), c.clone()
+        run(capi, gpu, prepared, a, b, one, 1.0, 0.5, out=one)
+        run(capi, gpu, plain, a, b, other, 1.0, 0.5, out=other)
+        assert torch.equal(one.view(torch.int32), other.view(torch.int32)), kind
+
+
+def test_a_plan_offers_both_forms(capi, gpu, oracle):
+    """Index 0 asks for the prepared form's workspace, the same Primitive without it follows, and index 0 still
+    runs with less."""
+    torch.manual_seed(3)
+    m = k = n = 2048
+    a, b = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda")
+    d = torch.empty(m, n, device="cuda")
+    plan = gpu.make_plan(a, b, None, d)
+    names = plan.primitive_names()
+    assert names[0] == names[1] and plan.workspace_bytes(0) > plan.workspace_bytes(1)
+    for index in (0, 1):
+        gpu.run_plan(plan, index)
+        check(oracle, d, a, b, None, 1.0, 0.0, f"index {index}")
+    less = torch.empty(max(plan.workspace_bytes(1), 1), dtype=torch.uint8, device="cuda")
+    plan.execute(0, less.data_ptr(), plan.workspace_bytes(1), gpu.current_stream())
+    torch.cuda.synchronize()
+    check(oracle, d, a, b, None, 1.0, 0.0, "index 0 with the minimum")
