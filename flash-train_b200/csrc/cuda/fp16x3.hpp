@@ -10,43 +10,52 @@
 namespace ftcuda {
 namespace fp16x3 {
 
-constexpr std::uint32_t kBlockK = 64;  // K elements of one block: 128 bytes of FP16, one swizzle row
+constexpr std::uint32_t kBlockK     = 64;   // K elements of one block: 128 bytes of FP16, one swizzle row
+constexpr std::uint32_t kSlabBlocks = 12;   // K blocks with scales of their own
+constexpr std::uint32_t kSlabK      = kSlabBlocks * kBlockK;
 
 // A split operand in the workspace: [rows][K blocks][high 64 | low 64] FP16, K-major whatever the
 // source's orientation, the last K block filled up with zeros.
 constexpr std::uint64_t kBlockBytes = 2 * kBlockK * 2;
 
-// Words at the head of the workspace, cleared in front of every launch.
-struct Control {
-    std::uint32_t use_fallback;  // the decision: 1 = this launch's operands go through the TF32 kernel
-    std::uint32_t out_of_range;  // a row or column whose largest magnitude the scaling does not cover
-    std::uint32_t gray;          // an element far below its row's (column's) largest was seen
-    std::uint32_t blocks_done;
-};
+// Rows of the operand that one CTA of the split takes, for one slab of K: source along K, or along the rows.
+constexpr std::uint32_t kSplitRowsAlongK = 16;
+constexpr std::uint32_t kSplitRows       = 32;
+
+constexpr std::uint32_t kColumnGroup = 16;  // columns of B that share a scale
+
+// What one CTA of the split found: how many elements of a row are below 2^-5, 2^-9 and 2^-13 of the largest
+// its scale allows for, in 1023rds of the slab (the worst row; ten bits each), an element far below that, a row
+// whose magnitudes the scaling does not cover.
+constexpr std::uint32_t kVerdictFew        = 0x3FF;
+constexpr std::uint32_t kVerdictGray       = 1U << 30;
+constexpr std::uint32_t kVerdictOutOfRange = 1U << 31;
 
 struct SplitOperand {
     const float* source;
     std::int64_t row_stride;  // between rows of A, or between columns of B
     std::int64_t k_stride;
     std::uint32_t rows;       // rows of A, or columns of B
+    std::uint32_t grouped;    // kColumnGroup rows share a scale, and `inverse` has one entry for each group
     std::uint32_t along_k;    // the source runs faster along K than along its rows
-    std::uint32_t vector;     // 16-byte loads along K are aligned
-    std::uint32_t max_blocks, split_blocks;  // CTAs of the two kernels that work on this operand
+    std::uint32_t vector;     // 16-byte loads in that direction are aligned
+    std::uint32_t blocks;     // CTAs
     unsigned char* split;
-    std::uint32_t* row_max;   // bit pattern of the largest magnitude of each row
-    std::uint32_t* few;       // elements of each row that are small against its largest
-    float* inverse;           // 1 / (scale of each row), a power of two
+    float* inverse;           // [slab][pitch]: 1 / (scale of the row or group in the slab), a power of two
+    std::uint64_t pitch;
+    std::uint32_t* verdicts;  // [blocks]
 };
 
 struct SplitParams {
     SplitOperand operand[2];
-    std::uint32_t k, k_blocks;
-    Control* control;
+    std::uint32_t k, k_blocks, slabs;
 };
 
-// CTAs of the two kernels for one operand.
-void planSplit(SplitOperand& operand, std::uint32_t k);
+// Fills along_k, vector and blocks from the source, its strides and the rows.
+void planSplit(SplitOperand& operand, std::uint32_t slabs);
 cudaError_t launchSplit(const SplitParams& params, cudaStream_t stream);
+// To be called once per process and device before launches (shared-memory size of the kernel).
+cudaError_t configureSplit();
 
 }  // namespace fp16x3
 }  // namespace ftcuda

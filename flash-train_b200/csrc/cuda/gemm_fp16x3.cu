@@ -1,7 +1,7 @@
 // The prepared form of the 3xTF32 families: D = alpha A B + beta C from operands split into FP16 pairs.
 //
 // A TF32 number and an FP16 number have the same 11 significant bits, and the tensor cores multiply
-// FP16 at twice the rate. With the operands scaled row by row (gemm_fp16x3_split.cu, which also says
+// FP16 at twice the rate. With the operands scaled (gemm_fp16x3_split.cu, which also says
 // when that is exact enough and leaves the launch to the TF32 kernel when it is not),
 //   a b = a_hi b_hi + (a_lo b_hi + a_hi b_lo) / 2^11,     a = a_hi + a_lo / 2^11, b likewise,
 // is three tcgen05.mma.kind::f16 products in half the tensor time of three TF32 ones, with less
@@ -12,27 +12,29 @@
 // A pair of CTAs (tcgen05 cta_group::2, a cluster of two) shares an output tile of 256 rows and up to
 // 256 columns, K walked in blocks of 64. Each CTA brings its 128 rows of A and half of the tile's rows
 // of B (B is K-major here whatever the caller's orientation), high and low parts, in two TMA copies:
-// at most 64 KiB a stage, three stages. One thread of the pair's first CTA issues the MMAs of both.
+// at most 64 KiB a stage, three stages.
 //
 //   warp 0       TMA producer (one thread, in both CTAs; the bytes of both count on the first CTA's barrier)
-//   warp 1       MMA issuer (one thread of the first CTA)
+//   warps 1, 2   MMA issuers (one thread each, in the first CTA, for both CTAs' tensor cores)
 //   warps 4-11   drain / epilogue, 32 rows x half of the columns each
 //
-// Tensor memory holds two accumulators, 512 columns in all: H (a_hi b_hi) and X (the two cross products).
-// The tensor core's FP32 additions truncate, so H is drained into registers every `chunk_blocks` K blocks
-// and added up there to nearest (see drainInterval in tf32x3_common.cuh); X, 2^11 times smaller in
-// effect, is read once per tile. In a K block the cross products are issued first: while the drain
-// warps read H, the tensor core works on the next block's eight MMAs into X, and at the end of a tile
-// X is read behind the last block's H products. The drain so costs the tensor pipe nothing; it cost
-// the TF32 kernel 4 %.
+// Tensor memory holds two accumulators, 512 columns in all: X, the two cross products, issued by warp 1, and H, a_hi b_hi,
+// issued by warp 2. Both are read at the end of every slab of K (768, the split's unit of scaling), multiplied by
+// the slab's powers of two -- exactly -- and added up in registers, to nearest. The tensor core's own FP32
+// additions truncate, so for a small K H is read more often than that (chunkBlocks); X is 2^11 times smaller
+// in effect. With an issuer each, one accumulator is read while products go to the other, and what a single thread does
+// between two K blocks -- barriers, descriptors -- no longer leaves the tensor pipe idle (one issuer for both:
+// 440 us instead of 388 at 4096^3, 187 instead of 154 at 2048 x 4096 x 3072). Rings of their own for the high and
+// the low parts, with H held one block behind X, were not faster (398 to 421 us).
 //
-// The epilogue turns each warp's 32 x 32 pieces in shared memory so that a row's 128 bytes are written
-// (and C's read) by eight neighbouring lanes, and undoes the scaling with the rows' and columns' powers
-// of two, exactly.
+// Shared memory is the resource next to the tensor pipe: operand fetches and TMA writes take 106 of its 128 bytes a
+// cycle. So the drain takes nothing from there -- B's scales are common to 16 columns and sit in registers -- and
+// the results go to memory straight from registers, 32 bytes a thread and store: 9400 cycles a tile, 15000 in pieces of
+// 16 bytes, 12000 turned in shared memory first (and the MMAs slower meanwhile).
 //
-// Measured, the whole launch with its split: 16384 x 4096 x 14336 8.81 -> 4.52 ms (218 -> 426 TFLOP/s; this kernel alone
-// 499, three times that in FP16 products, 0.91 of the measured dense BF16 rate: what bounds it is the power limit),
-// 4096^3 688 -> 471 us.
+// Measured, the whole launch with its split, TF32 form / this one in microseconds: 16384 x 4096 x 14336 8850 / 4600 (up
+// to 426 TFLOP/s; what bounds it is the power limit: the products alone run at 0.91 of the measured dense BF16
+// rate), 8192 x 4096 x 8192 2780 / 1440, 4096^3 710 / 400, 2048^3 115 / 63, 1024 x 1024 x 4096 83 / 39.
 //
 // Every wait is bounded, as in the other kernels (ptx.cuh).
 #include <cuda.h>
@@ -48,18 +50,17 @@
 namespace ftcuda {
 namespace {
 
-using fp16x3::Control;
 using fp16x3::kBlockBytes;
 using fp16x3::kBlockK;
+using fp16x3::kSlabBlocks;
 
 constexpr int kTileM      = 256;  // of a CTA pair
 constexpr int kMaxTileN   = 256;
 constexpr int kStages     = 3;
 constexpr int kThreads    = 384;
-constexpr int kABytes     = 128 * static_cast<int>(kBlockBytes);          // hi | lo, 16 KiB each
-constexpr int kStageBytes = kABytes + kMaxTileN / 2 * static_cast<int>(kBlockBytes);
-constexpr int kTurnOffset = kStages * kStageBytes;                        // 4 KiB per epilogue warp
-constexpr int kBarrierOffset = kTurnOffset + 8 * 4096;
+constexpr int kABytes     = 128 * static_cast<int>(kBlockBytes);  // a CTA's A tile: high | low, 16 KiB each
+constexpr int kStageBytes = kABytes + kMaxTileN / 2 * static_cast<int>(kBlockBytes);  // ... and its half of B's
+constexpr int kBarrierOffset = kStages * kStageBytes;
 constexpr int kSmemBytes     = kBarrierOffset + 256 + 1024;
 static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
 
@@ -67,19 +68,21 @@ constexpr int kRegsLight = 72;   // producer, issuer (warpgroup 0)
 constexpr int kRegsDrain = 216;  // drain / epilogue (warpgroups 1, 2)
 static_assert(128 * kRegsLight + 256 * kRegsDrain <= 168 * kThreads, "the CTA's register pool is what it was launched with");
 constexpr int kProducerWarp  = 0;
-constexpr int kMmaWarp       = 1;
+constexpr int kCrossWarp     = 1;
+constexpr int kHighWarp      = 2;
 constexpr int kFirstEpilogue = 4;
 constexpr std::uint32_t kTmemColumns = 512;
 constexpr std::uint32_t kHColumn     = 256;  // X at 0
 
 struct Barriers {
-    std::uint64_t full[kStages];   // used in the pair's first CTA
+    std::uint64_t full[kStages];  // used in the pair's first CTA
     std::uint64_t empty[kStages];
     std::uint64_t x_full, h_full;
     std::uint64_t x_empty, h_empty;  // used in the pair's first CTA
-    std::uint64_t flush;
+    std::uint64_t flush_x, flush_h;
     std::uint32_t tmem_base;
     int abort_flag;
+    std::uint32_t few[2][3], flags;  // the worst of the verdicts
 };
 static_assert(sizeof(Barriers) <= 256, "barrier block");
 
@@ -93,11 +96,14 @@ struct Fp16Params {
     std::uint32_t tiles_m, tiles_n, tile_n, band_m_tiles;
     std::uint32_t chunk_blocks;
     float alpha, beta;
-    float* partials;  // non-null: unscaled sums of the K slices, [split][m][n]
-    const float* inverse_a;
+    float* partials;  // non-null: the K slices' sums, [split][m][n]
+    const float* inverse_a;  // [slab][inverse_pitch_a]
     const float* inverse_b;
-    const Control* control;
-    std::uint32_t vector;  // 16-byte accesses to the output and to C are aligned
+    std::uint64_t inverse_pitch_a, inverse_pitch_b;
+    const std::uint32_t* verdicts;  // of the split's CTAs: first A's, then B's
+    std::uint32_t verdicts_a, verdicts_b;
+    std::uint32_t* use_fallback;    // the decision, for the kernels behind this one
+    std::uint32_t vector;  // consecutive columns of the output and C that one aligned access takes: 8, 4, or 0 (any strides)
     int* status;
 };
 
@@ -121,65 +127,121 @@ __device__ __forceinline__ Item decode(const Fp16Params& p, std::uint32_t item) 
     return w;
 }
 
-// Rows and columns of one warp's share, written 32 columns at a time.
-__device__ __forceinline__ void writePiece(const Fp16Params& p, const Item& w, std::uint32_t row0, std::uint32_t col0,
-                                           unsigned char* turn, int lane, const float* values) {
-    // A thread holds 32 columns of its row; 16-byte chunks are stored XOR-ed with the row so that
-    // neither side of the turn has bank conflicts.
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        *reinterpret_cast<float4*>(turn + lane * 128 + ((c ^ (lane & 7)) << 4)) =
-            make_float4(values[4 * c], values[4 * c + 1], values[4 * c + 2], values[4 * c + 3]);
+// Position in a ring of slots: the slot, and how often the ring has been gone round.
+struct Ring {
+    std::uint32_t slots, slot = 0, round = 0;
+    __device__ __forceinline__ explicit Ring(std::uint32_t n) : slots(n) {}
+    __device__ __forceinline__ void next() {
+        if (++slot == slots) {
+            slot = 0;
+            ++round;
+        }
     }
-    __syncwarp();
-    const std::uint32_t col = col0 + (lane & 7) * 4;
-    float cs[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { cs[j] = col + j < p.n ? p.inverse_b[col + j] : 0.0F; }
-    const bool partial = p.partials != nullptr;
-    float* const out   = partial ? p.partials + static_cast<std::uint64_t>(w.split) * p.m * p.n : p.d;
+};
+
+// K blocks of an item from `block` on that lie in one slab. (A K slice may begin and end inside one.)
+__device__ __forceinline__ std::uint32_t blocksInSlab(const Item& w, std::uint32_t block) {
+    return min(kSlabBlocks - (w.first_block + block) % kSlabBlocks, w.blocks - block);
+}
+
+// Writes 32 consecutive columns of one row, held by one thread.
+__device__ __forceinline__ void writePiece(const Fp16Params& p, const Item& w, std::uint32_t row, std::uint32_t col, const float2* values) {
+    const std::uint32_t end       = min(p.n, w.col + p.tile_n);  // of the tile's columns
+    const bool partial            = p.partials != nullptr;
+    float* const out              = partial ? p.partials + static_cast<std::uint64_t>(w.split) * p.m * p.n : p.d;
     const std::int64_t row_stride = partial ? p.n : p.d_row_stride;
-    const std::int64_t col_stride = partial ? 1 : p.d_col_stride;
     const float* const c          = partial ? nullptr : p.c;
     const float alpha             = partial ? 1.0F : p.alpha;
-    const bool vector             = p.vector != 0 && col + 4 <= p.n;
+    if (p.vector == 8) {
+        // 32 bytes, a whole sector, per thread and store: half the passes through the L1 that 16 take.
+        float* const at = out + static_cast<std::int64_t>(row) * row_stride + col;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r             = i * 4 + (lane >> 3);
-        const std::uint32_t row = row0 + r;
-        const float4 v = *reinterpret_cast<const float4*>(turn + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
-        if (row >= p.m) { continue; }
-        float o[4] = {v.x * cs[0] * alpha, v.y * cs[1] * alpha, v.z * cs[2] * alpha, v.w * cs[3] * alpha};
-        float* const at = out + static_cast<std::int64_t>(row) * row_stride + static_cast<std::int64_t>(col) * col_stride;
-        if (vector) {
+        for (int half = 0; half < 2; ++half) {
+            float addend[2][8];
             if (c != nullptr) {
-                const float4 addend = *reinterpret_cast<const float4*>(c + static_cast<std::int64_t>(row) * p.c_row_stride + col);
-                o[0] += p.beta * addend.x;
-                o[1] += p.beta * addend.y;
-                o[2] += p.beta * addend.z;
-                o[3] += p.beta * addend.w;
-            }
-            *reinterpret_cast<float4*>(at) = make_float4(o[0], o[1], o[2], o[3]);
-        } else {
+                // C's values are asked for before the stores: C may be D, so the compiler moves no load past a store by itself.
+                const float* const from = c + static_cast<std::int64_t>(row) * p.c_row_stride + col + 16 * half;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (col + j >= p.n) { continue; }
-                if (c != nullptr) {
-                    o[j] += p.beta * c[static_cast<std::int64_t>(row) * p.c_row_stride + static_cast<std::int64_t>(col + j) * p.c_col_stride];
+                for (int j = 0; j < 2; ++j) {
+                    if (col + 16 * half + 8 * j < end) { loadGlobal8(from + 8 * j, addend[j]); }
                 }
-                at[j * col_stride] = o[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if (col + 16 * half + 8 * j >= end) { continue; }
+                float o[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    o[2 * i]     = alpha * values[8 * half + 4 * j + i].x;
+                    o[2 * i + 1] = alpha * values[8 * half + 4 * j + i].y;
+                }
+                if (c != nullptr) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { o[i] += p.beta * addend[j][i]; }
+                }
+                storeGlobal8(at + 16 * half + 8 * j, o);
+            }
+        }
+        return;
+    }
+    if (p.vector == 4) {
+        float* const at         = out + static_cast<std::int64_t>(row) * row_stride + col;
+        const float* const from = c != nullptr ? c + static_cast<std::int64_t>(row) * p.c_row_stride + col : nullptr;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (col + 4 * j >= end) { continue; }
+            const float2 low = values[2 * j], high = values[2 * j + 1];
+            float4 o = make_float4(alpha * low.x, alpha * low.y, alpha * high.x, alpha * high.y);
+            if (c != nullptr) {
+                const float4 addend = *reinterpret_cast<const float4*>(from + 4 * j);
+                o.x += p.beta * addend.x;
+                o.y += p.beta * addend.y;
+                o.z += p.beta * addend.z;
+                o.w += p.beta * addend.w;
+            }
+            *reinterpret_cast<float4*>(at + 4 * j) = o;
+        }
+        return;
+    }
+    const std::int64_t col_stride = partial ? 1 : p.d_col_stride;
+    float* const at = out + static_cast<std::int64_t>(row) * row_stride + static_cast<std::int64_t>(col) * col_stride;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        if (col + j >= end) { continue; }
+        float value = alpha * (j % 2 == 0 ? values[j / 2].x : values[j / 2].y);
+        if (c != nullptr) {
+            value += p.beta * c[static_cast<std::int64_t>(row) * p.c_row_stride + static_cast<std::int64_t>(col + j) * p.c_col_stride];
+        }
+        at[j * col_stride] = value;
+    }
+}
+
+// acc += row_scale * scale of the 16 columns * accumulator, for up to four pieces of 32 columns at `tmem`. The products
+// of powers of two are exact.
+__device__ __forceinline__ void addScaled(std::uint32_t tmem, std::uint32_t pieces, float row_scale, const float (&scales)[8],
+                                          float2 (&acc)[64]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (static_cast<std::uint32_t>(q) < pieces) {
+            float v[32];
+            tmemLoad32(tmem + q * 32, v);
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                const float scale = row_scale * scales[2 * q + g];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    float2& sum = acc[q * 16 + g * 8 + j];
+                    sum = multiplyAdd2(make_float2(scale, scale), make_float2(v[g * 16 + 2 * j], v[g * 16 + 2 * j + 1]), sum);
+                }
             }
         }
     }
-    __syncwarp();
 }
 
 __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
 tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Fp16Params p,
-                 const std::uint32_t num_items) {
+                 std::uint32_t num_items) {
     extern __shared__ unsigned char smem_raw[];
-    // The decision of the split: every CTA leaves together.
-    if (p.control->use_fallback != 0) { return; }
     const std::uint32_t align_offset = (1024 - (smemAddress(smem_raw) & 1023)) & 1023;
     unsigned char* smem              = smem_raw + align_offset;
     Barriers* bars                   = reinterpret_cast<Barriers*>(smem + kBarrierOffset);
@@ -193,19 +255,22 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbarrierInit(&bars->full[s], 1);
-            mbarrierInit(&bars->empty[s], 1);
+            mbarrierInit(&bars->empty[s], 2);  // both issuers
         }
         mbarrierInit(&bars->x_full, 1);
         mbarrierInit(&bars->h_full, 1);
         mbarrierInit(&bars->x_empty, 16);
         mbarrierInit(&bars->h_empty, 16);
-        mbarrierInit(&bars->flush, 1);
+        mbarrierInit(&bars->flush_x, 1);
+        mbarrierInit(&bars->flush_h, 1);
         bars->abort_flag = 0;
+        for (int i = 0; i < 6; ++i) { bars->few[i / 3][i % 3] = 0; }
+        bars->flags = 0;
         fenceBarrierInit();
         prefetchTensorMap(&map_a);
         prefetchTensorMap(&map_b);
     }
-    if (warp == kMmaWarp) { tmemAllocatePair(&bars->tmem_base, kTmemColumns); }
+    if (warp == kCrossWarp) { tmemAllocatePair(&bars->tmem_base, kTmemColumns); }
     tcgen05FenceBeforeSync();
     __syncthreads();
     clusterBarrierArrive();
@@ -213,70 +278,96 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     tcgen05FenceAfterSync();
     const std::uint32_t tmem_base = bars->tmem_base;
 
+    // Launched with programmatic stream serialization: what is above overlaps the split's tail.
+    gridDependencyWait();
+    gridDependencyLaunchDependents();
+    // Every CTA comes to the same decision. Left to the fallback, there are no items.
+    {
+        std::uint32_t flags = 0;
+        for (int which = 0; which < 2; ++which) {
+            const std::uint32_t* const verdicts = p.verdicts + (which != 0 ? p.verdicts_a : 0);
+            const std::uint32_t count           = which != 0 ? p.verdicts_b : p.verdicts_a;
+            std::uint32_t few[3]                = {0, 0, 0};
+#pragma unroll 4
+            for (std::uint32_t i = threadIdx.x; i < count; i += kThreads) {
+                const std::uint32_t verdict = __ldcg(verdicts + i);
+                flags |= verdict;
+#pragma unroll
+                for (int t = 0; t < 3; ++t) { few[t] = max(few[t], verdict >> (10 * t) & fp16x3::kVerdictFew); }
+            }
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                few[t] = __reduce_max_sync(0xFFFFFFFFU, few[t]);
+                if (lane == 0) { atomicMax(&bars->few[which][t], few[t]); }
+            }
+        }
+        flags = __reduce_or_sync(0xFFFFFFFFU, flags);
+        if (lane == 0) { atomicOr(&bars->flags, flags); }
+        __syncthreads();
+        // F_a + F_b - 1 >= 1/64, in 1023rds of a slab and with one to spare for the rounding of each, for any pair
+        // of thresholds whose exponents add up to 18.
+        const auto enough = [&](int a, int b) { return bars->few[0][a] + bars->few[1][b] + 16 + 2 <= 1023; };
+        const bool fallback = (bars->flags & fp16x3::kVerdictOutOfRange) != 0 ||
+                              ((bars->flags & fp16x3::kVerdictGray) != 0 && !enough(0, 2) && !enough(1, 1) && !enough(2, 0));
+        if (blockIdx.x == 0 && threadIdx.x == 0) { *p.use_fallback = fallback ? 1U : 0U; }
+        if (fallback) { num_items = 0; }
+    }
+
     if (warp >= kFirstEpilogue) {
         registersGrow<kRegsDrain>();
-        const int e                   = warp - kFirstEpilogue;  // 0..7; warp % 4 is the tensor-memory lane quadrant
-        const std::uint32_t in_tile   = static_cast<std::uint32_t>(32 * (e & 3));
+        const int e                   = warp - kFirstEpilogue;                    // 0..7
+        const std::uint32_t in_tile   = static_cast<std::uint32_t>(32 * (warp & 3));  // the tensor-memory lanes a warp can read
         const std::uint32_t tmem_row  = tmem_base + (in_tile << 16);
-        const std::uint32_t pieces    = p.tile_n / 32;
+        const std::uint32_t pieces    = (p.tile_n + 31) / 32;
         const std::uint32_t first     = (e >> 2) != 0 ? (pieces + 1) / 2 : 0;  // this warp's pieces of 32 columns
         const std::uint32_t mine      = (e >> 2) != 0 ? pieces / 2 : (pieces + 1) / 2;
-        unsigned char* turn           = smem + kTurnOffset + e * 4096;
         const std::uint32_t x_empty   = mapToRank(&bars->x_empty, 0);
         const std::uint32_t h_empty   = mapToRank(&bars->h_empty, 0);
-        std::uint32_t items = 0, chunks = 0;
+        std::uint32_t slabs = 0, chunks = 0;
         bool ok = true;
-        for (std::uint32_t item = pair; item < num_items && ok; item += pairs, ++items) {
-            const Item w                   = decode(p, item);
-            const std::uint32_t num_chunks = (w.blocks + p.chunk_blocks - 1) / p.chunk_blocks;
-            float acc[128];
+        for (std::uint32_t item = pair; item < num_items && ok; item += pairs) {
+            const Item w             = decode(p, item);
+            const std::uint32_t row0 = w.row + rank * 128 + in_tile;
+            const std::uint32_t mine_at = w.col + first * 32;
+            float2 acc[64];
 #pragma unroll
-            for (int j = 0; j < 128; ++j) { acc[j] = 0.0F; }
-            for (std::uint32_t chunk = 0; chunk < num_chunks && ok; ++chunk, ++chunks) {
-                if (chunk + 1 == num_chunks) {
-                    ok = mbarrierWait(&bars->x_full, items & 1, abort_flag);
+            for (int j = 0; j < 64; ++j) { acc[j] = make_float2(0.0F, 0.0F); }
+            for (std::uint32_t block = 0, in_slab; block < w.blocks && ok; block += in_slab, ++slabs) {
+                in_slab = blocksInSlab(w, block);
+                // The slab's scales: of this thread's row, and of this warp's groups of 16 columns.
+                const std::uint32_t slab = (w.first_block + block) / kSlabBlocks;
+                const float row_scale    = p.inverse_a[slab * p.inverse_pitch_a + row0 + lane];
+                const float* const groups = p.inverse_b + slab * p.inverse_pitch_b + mine_at / fp16x3::kColumnGroup;
+                float scales[8];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) { scales[g] = groups[g]; }
+                const std::uint32_t num_chunks = (in_slab + p.chunk_blocks - 1) / p.chunk_blocks;
+                for (std::uint32_t chunk = 0; chunk < num_chunks && ok; ++chunk, ++chunks) {
+                    // X once per slab, ahead of the last reading of H.
+                    if (chunk + 1 == num_chunks) {
+                        ok = mbarrierWait(&bars->x_full, slabs & 1, abort_flag);
+                        if (!ok) { break; }
+                        tcgen05FenceAfterSync();
+                        addScaled(tmem_row + first * 32, mine, row_scale * 0x1p-11F, scales, acc);
+                        tcgen05FenceBeforeSync();
+                        __syncwarp();
+                        if (lane == 0) { mbarrierArriveCluster(x_empty); }
+                    }
+                    ok = mbarrierWait(&bars->h_full, chunks & 1, abort_flag);
                     if (!ok) { break; }
                     tcgen05FenceAfterSync();
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        if (static_cast<std::uint32_t>(q) < mine) {
-                            float x[32];
-                            tmemLoad32(tmem_row + (first + q) * 32, x);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) { acc[q * 32 + j] += x[j] * 0x1p-11F; }
-                        }
-                    }
+                    addScaled(tmem_row + kHColumn + first * 32, mine, row_scale, scales, acc);
                     tcgen05FenceBeforeSync();
                     __syncwarp();
-                    if (lane == 0) { mbarrierArriveCluster(x_empty); }
+                    if (lane == 0) { mbarrierArriveCluster(h_empty); }
                 }
-                ok = mbarrierWait(&bars->h_full, chunks & 1, abort_flag);
-                if (!ok) { break; }
-                tcgen05FenceAfterSync();
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (static_cast<std::uint32_t>(q) < mine) {
-                        float h[32];
-                        tmemLoad32(tmem_row + kHColumn + (first + q) * 32, h);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) { acc[q * 32 + j] += h[j]; }
-                    }
-                }
-                tcgen05FenceBeforeSync();
-                __syncwarp();
-                if (lane == 0) { mbarrierArriveCluster(h_empty); }
             }
             if (!ok) { break; }
-            const std::uint32_t row0 = w.row + rank * 128 + in_tile;
-            const std::uint32_t row  = row0 + lane;
-            const float row_scale    = row < p.m ? p.inverse_a[row] : 0.0F;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const std::uint32_t col0 = w.col + (first + q) * 32;
-                if (static_cast<std::uint32_t>(q) < mine && col0 < p.n && row0 < p.m) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) { acc[q * 32 + j] *= row_scale; }
-                    writePiece(p, w, row0, col0, turn, lane, acc + q * 32);
+                const std::uint32_t col = mine_at + q * 32;
+                if (static_cast<std::uint32_t>(q) < mine && col < p.n && row0 + lane < p.m) {
+                    writePiece(p, w, row0 + lane, col, acc + q * 16);
                 }
             }
         }
@@ -287,28 +378,23 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             bool ok = true;
             if (lane == 0) {
                 const std::uint32_t stage_bytes = kABytes + p.tile_n / 2 * static_cast<std::uint32_t>(kBlockBytes);
-                std::uint32_t s = 0, parity = 1;
+                Ring ring(kStages);
                 std::uint32_t filled = 0;
                 for (std::uint32_t item = pair; item < num_items && ok; item += pairs) {
                     const Item w = decode(p, item);
                     const std::int32_t row_a = static_cast<std::int32_t>(w.row + rank * 128);
                     const std::int32_t row_b = static_cast<std::int32_t>(w.col + rank * (p.tile_n / 2));
-                    for (std::uint32_t kb = 0; kb < w.blocks; ++kb) {
-                        ok = mbarrierWait(&bars->empty[s], parity, abort_flag);
+                    for (std::uint32_t kb = 0; kb < w.blocks; ++kb, ++filled, ring.next()) {
+                        ok = mbarrierWait(&bars->empty[ring.slot], (ring.round & 1) ^ 1, abort_flag);
                         if (!ok) { break; }
                         // The bytes of both CTAs count on the first CTA's barrier, which that CTA arms. (The other's
                         // may land first: the phase cannot complete before it has been armed.)
-                        if (rank == 0) { mbarrierArriveExpectTx(&bars->full[s], 2 * stage_bytes); }
-                        const std::uint32_t full  = mapToRank(&bars->full[s], 0);
-                        unsigned char* const slot = smem + s * kStageBytes;
+                        if (rank == 0) { mbarrierArriveExpectTx(&bars->full[ring.slot], 2 * stage_bytes); }
+                        const std::uint32_t full  = mapToRank(&bars->full[ring.slot], 0);
+                        unsigned char* const slot = smem + ring.slot * kStageBytes;
                         const std::int32_t z      = static_cast<std::int32_t>((w.first_block + kb) * 2);
                         tmaLoad3dPair(slot, &map_a, full, 0, row_a, z);
                         tmaLoad3dPair(slot + kABytes, &map_b, full, 0, row_b, z);
-                        ++filled;
-                        if (++s == kStages) {
-                            s = 0;
-                            parity ^= 1;
-                        }
                     }
                 }
                 // Neither CTA leaves before the last commits have arrived on its barriers.
@@ -319,61 +405,61 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (!ok) { *abort_flag = 1; }
             }
             __syncwarp();
-        } else if (warp == kMmaWarp && rank == 0) {
+        } else if ((warp == kCrossWarp || warp == kHighWarp) && rank == 0) {
             if (lane == 0) {
+                const bool cross                = warp == kCrossWarp;
                 const std::uint32_t instruction = umaInstructionF16(kTileM, p.tile_n);
-                const std::uint32_t b_low       = p.tile_n / 2 * 128;  // bytes of B's high part in a stage
-                std::uint32_t s = 0, parity = 0;
-                std::uint32_t items = 0, chunks = 0;
-                bool ok = true;
-                for (std::uint32_t item = pair; item < num_items && ok; item += pairs, ++items) {
-                    const Item w           = decode(p, item);
-                    std::uint32_t in_chunk = 0;
-                    for (std::uint32_t kb = 0; kb < w.blocks; ++kb) {
-                        const bool last = kb + 1 == w.blocks;
-                        if (kb == 0) { ok = mbarrierWait(&bars->x_empty, (items & 1) ^ 1, abort_flag); }
-                        ok = ok && mbarrierWait(&bars->full[s], parity, abort_flag);
+                // Operand descriptors of the first stage, and their distance to the next, in units of 16 bytes.
+                const std::uint64_t stage_step = kStageBytes >> 4;
+                const std::uint64_t a_hi0 = umaDescriptorK128(smemAddress(smem)), a_lo0 = a_hi0 + (128 * 128 >> 4);
+                const std::uint64_t b_hi0 = a_hi0 + (kABytes >> 4), b_lo0 = b_hi0 + (p.tile_n / 2 * 128 >> 4);
+                std::uint64_t* const sum_full  = cross ? &bars->x_full : &bars->h_full;
+                std::uint64_t* const sum_empty = cross ? &bars->x_empty : &bars->h_empty;
+                Ring ring(kStages);
+                std::uint32_t sums = 0;
+                bool ok            = true;
+                for (std::uint32_t item = pair; item < num_items && ok; item += pairs) {
+                    const Item w = decode(p, item);
+                    // K blocks left in the slab, and in the sum that goes to the drain warps next.
+                    std::uint32_t in_slab = 0, in_sum = 0;
+                    for (std::uint32_t kb = 0; kb < w.blocks; ++kb, ring.next()) {
+                        if (in_slab == 0) { in_slab = blocksInSlab(w, kb); }
+                        const bool fresh = in_sum == 0;
+                        if (fresh) {
+                            in_sum = cross ? in_slab : min(in_slab, p.chunk_blocks);
+                            ok     = mbarrierWait(sum_empty, (sums & 1) ^ 1, abort_flag);
+                            if (!ok) { break; }
+                            ++sums;
+                        }
+                        ok = mbarrierWait(&bars->full[ring.slot], ring.round & 1, abort_flag);
                         if (!ok) { break; }
                         tcgen05FenceAfterSync();
-                        const std::uint32_t slot  = smemAddress(smem + s * kStageBytes);
-                        const std::uint64_t a_hi  = umaDescriptorK128(slot);
-                        const std::uint64_t a_lo  = umaDescriptorK128(slot + 128 * 128);
-                        const std::uint64_t b_hi  = umaDescriptorK128(slot + kABytes);
-                        const std::uint64_t b_lo  = umaDescriptorK128(slot + kABytes + b_low);
+                        const std::uint64_t a_hi = a_hi0 + ring.slot * stage_step, b_hi = b_hi0 + ring.slot * stage_step;
+                        if (cross) {
+                            const std::uint64_t a_lo = a_lo0 + ring.slot * stage_step, b_lo = b_lo0 + ring.slot * stage_step;
 #pragma unroll
-                        for (std::uint32_t step = 0; step < kBlockK / 16; ++step) {  // 32 bytes along K = two descriptor units
-                            umaF16Pair(tmem_base, a_lo + 2 * step, b_hi + 2 * step, instruction, kb != 0 || step != 0 ? 1U : 0U);
-                            umaF16Pair(tmem_base, a_hi + 2 * step, b_lo + 2 * step, instruction, 1U);
-                        }
-                        if (last) { umaCommitPair(&bars->x_full); }
-                        if (in_chunk == 0) {
-                            ok = mbarrierWait(&bars->h_empty, (chunks & 1) ^ 1, abort_flag);
-                            if (!ok) { break; }
-                            tcgen05FenceAfterSync();
-                            ++chunks;
-                        }
+                            for (std::uint32_t step = 0; step < kBlockK / 16; ++step) {  // 32 bytes along K = two descriptor units
+                                umaF16Pair(tmem_base, a_lo + 2 * step, b_hi + 2 * step, instruction, !fresh || step != 0 ? 1U : 0U);
+                                umaF16Pair(tmem_base, a_hi + 2 * step, b_lo + 2 * step, instruction, 1U);
+                            }
+                        } else {
 #pragma unroll
-                        for (std::uint32_t step = 0; step < kBlockK / 16; ++step) {
-                            umaF16Pair(tmem_base + kHColumn, a_hi + 2 * step, b_hi + 2 * step, instruction,
-                                       in_chunk != 0 || step != 0 ? 1U : 0U);
+                            for (std::uint32_t step = 0; step < kBlockK / 16; ++step) {
+                                umaF16Pair(tmem_base + kHColumn, a_hi + 2 * step, b_hi + 2 * step, instruction, !fresh || step != 0 ? 1U : 0U);
+                            }
                         }
-                        umaCommitPair(&bars->empty[s]);
-                        if (++in_chunk == p.chunk_blocks || last) {
-                            umaCommitPair(&bars->h_full);
-                            in_chunk = 0;
-                        }
-                        if (++s == kStages) {
-                            s = 0;
-                            parity ^= 1;
-                        }
+                        umaCommitPair(&bars->empty[ring.slot]);
+                        --in_slab;
+                        if (--in_sum == 0) { umaCommitPair(sum_full); }
                     }
                 }
                 if (!ok) {
                     *abort_flag = 1;
                     // Let MMAs already issued finish before tensor memory is freed.
-                    umaCommitPair(&bars->flush);
+                    std::uint64_t* const flush = cross ? &bars->flush_x : &bars->flush_h;
+                    umaCommitPair(flush);
                     int never = 0;
-                    mbarrierWait(&bars->flush, 0, &never);
+                    mbarrierWait(flush, 0, &never);
                 }
             }
             __syncwarp();
@@ -397,21 +483,36 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     tcgen05FenceBeforeSync();
     clusterBarrierArrive();
     clusterBarrierWait();
-    if (warp == kMmaWarp) {
+    if (warp == kCrossWarp) {
         tcgen05FenceAfterSync();
         tmemFreePair(tmem_base, kTmemColumns);
     }
 }
 
-// K blocks (of 64) accumulated into H between two drains. A block is four truncating additions where the TF32 kernel
-// makes twelve for half of the depth. Relative error against float64 at K = 4096: 4.3e-7 with a drain every 5
-// blocks, 7.8e-7 every 10 (the choice there), 1.14e-6 every 15, 4.9e-6 never; the TF32 kernel 1.13e-6. The time
-// does not depend on it (447, 445, 462, 428 us).
-std::uint32_t preparedChunkBlocks(std::uint64_t k) {
-    return 2 * tf32x3::drainInterval(k);
+// K blocks (of 64) accumulated into H between two drains, a divisor of the slab's. A block is four truncating
+// additions where the TF32 kernel makes twelve for half of the depth, so up to three times its interval of
+// blocks of 32 has no more of them in a row.
+std::uint32_t chunkBlocks(std::uint64_t k) {
+    const std::uint32_t interval = tf32x3::drainInterval(k);
+    return interval >= 4 ? 12 : interval >= 2 ? 6 : 2;
 }
 
 std::uint64_t roundUp(std::uint64_t x, std::uint64_t unit) { return (x + unit - 1) / unit * unit; }
+
+// A's rows and B's columns as the split sees them.
+void describeOperands(const FtcudaGemmDesc& desc, fp16x3::SplitOperand (&operands)[2]) {
+    operands[0]            = {};
+    operands[0].source     = desc.a;
+    operands[0].row_stride = desc.a_row_stride;
+    operands[0].k_stride   = desc.a_col_stride;
+    operands[0].rows       = static_cast<std::uint32_t>(desc.m);
+    operands[1]            = {};
+    operands[1].source     = desc.b;
+    operands[1].row_stride = desc.b_col_stride;
+    operands[1].k_stride   = desc.b_row_stride;
+    operands[1].rows       = static_cast<std::uint32_t>(desc.n);
+    operands[1].grouped    = 1;
+}
 
 // Tile width and K slices. Modelled cost in SM cycles: a K step of 16 is three MMAs of tile_n / 2 cycles each, or the
 // shared-memory traffic behind them (operand fetches and TMA writes at 128 bytes a cycle) where that is longer, which it is
@@ -424,14 +525,14 @@ struct Geometry {
 
 Geometry chooseGeometry(std::uint64_t m, std::uint64_t n, std::uint64_t k_blocks, std::uint64_t pairs) {
     Geometry best{kMaxTileN, 1, static_cast<std::uint32_t>(k_blocks), 0.0};
-    for (std::uint32_t width = kMaxTileN; width >= 64; width -= 32) {
+    for (std::uint32_t width = kMaxTileN; width >= 64; width -= 16) {
         const std::uint64_t tiles = ceilDiv(m, kTileM) * ceilDiv(n, width);
         const double mma          = 1.5 * width;
         const double smem         = 160.0 + 0.625 * width;
         const double block_cycles = 4.0 * (mma > smem ? mma : smem);
         for (std::uint32_t splits = 1; splits <= 32; ++splits) {
-            const std::uint64_t per_split = ceilDiv(k_blocks, splits);
-            if (splits > 1 && (per_split < 4 || ceilDiv(k_blocks, per_split) != splits)) { continue; }
+            const std::uint64_t per_split = splits == 1 ? k_blocks : roundUp(ceilDiv(k_blocks, splits), 4);
+            if (splits > 1 && ( ceilDiv(k_blocks, per_split) != splits)) { continue; }
             if (tiles * splits >= (1ULL << 31)) { break; }
             double cycles = static_cast<double>(ceilDiv(tiles * splits, pairs)) * (static_cast<double>(per_split) * block_cycles + 4000.0);
             if (splits > 1) { cycles += 8000.0 + static_cast<double>(m) * static_cast<double>(n) * (8.0 * splits + 4.0) / 3500.0; }
@@ -466,32 +567,32 @@ int configurePrepared(LaunchState& state, const FtcudaGemmDesc& desc, char* mess
     prepared.tile_n              = geometry.tile_n;
     prepared.splits              = geometry.splits;
     prepared.blocks_per_split    = geometry.blocks_per_split;
-    prepared.chunk_blocks        = preparedChunkBlocks(desc.k);
+    prepared.chunk_blocks        = chunkBlocks(desc.k);
     const std::uint64_t items    = ceilDiv(desc.m, kTileM) * ceilDiv(desc.n, geometry.tile_n) * geometry.splits;
     prepared.grid                = static_cast<std::uint32_t>(2 * (items < pairs ? items : pairs));
 
     const std::uint64_t rows[2] = {desc.m, desc.n};
-    std::uint64_t at            = 256;  // Control
+    const std::uint64_t slabs   = ceilDiv(k_blocks, kSlabBlocks);
+    fp16x3::SplitOperand operands[2];
+    describeOperands(desc, operands);
+    for (fp16x3::SplitOperand& operand : operands) { fp16x3::planSplit(operand, static_cast<std::uint32_t>(slabs)); }
+    std::uint64_t at            = 256;  // the decision
+    prepared.verdicts_at        = at;
+    at += roundUp((static_cast<std::uint64_t>(operands[0].blocks) + operands[1].blocks) * 4, 256);
     for (int i = 0; i < 2; ++i) {
-        prepared.max_at[i] = at;
-        at += roundUp(rows[i] * 4, 256);
-        prepared.few_at[i] = at;
-        at += roundUp(rows[i] * 4, 256);
+        // A tile reads its scales beyond the last row, too (and does not use them).
+        prepared.inverse_pitch[i] = roundUp((rows[i] + 2 * kMaxTileN) / (i == 0 ? 1 : fp16x3::kColumnGroup), 4);
+        prepared.inverse_at[i]    = at;
+        at += roundUp(slabs * prepared.inverse_pitch[i] * 4, 256);
     }
-    prepared.cleared_bytes = at;
-    for (int i = 0; i < 2; ++i) {
-        prepared.inverse_at[i] = at;
-        at += roundUp(rows[i] * 4, 256);
-    }
-    const std::uint64_t control_bytes = at;
     for (int i = 0; i < 2; ++i) {
         prepared.split_at[i] = at;
         at += roundUp(rows[i] * k_blocks * kBlockBytes, 256);
     }
     prepared.partials_at = at;
     if (prepared.splits > 1) { at += static_cast<std::uint64_t>(prepared.splits) * desc.m * desc.n * sizeof(float); }
-    // The fallback's own workspace lies over the split operands, which it does not need.
-    const std::uint64_t fallback = control_bytes + state.workspace_bytes;
+    // The fallback's own workspace lies over all of this but the decision: it runs when none of it is needed any more.
+    const std::uint64_t fallback = 256 + state.workspace_bytes;
     state.workspace_bytes        = (at > fallback ? at : fallback) + 256;
 
     // Encoded for a stand-in address; re-pointed at the workspace in front of every launch.
@@ -500,7 +601,8 @@ int configurePrepared(LaunchState& state, const FtcudaGemmDesc& desc, char* mess
         !encodeSplitMap(&prepared.map_b, stand_in, desc.n, k_blocks, prepared.tile_n / 2, message, capacity)) {
         return 1;
     }
-    const cudaError_t error = cudaFuncSetAttribute(tensorGemm3xFp16, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    cudaError_t error = cudaFuncSetAttribute(tensorGemm3xFp16, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (error == cudaSuccess) { error = fp16x3::configureSplit(); }
     if (error != cudaSuccess) { return fail(message, capacity, 1, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(error)); }
     return 0;
 }
@@ -509,32 +611,23 @@ cudaError_t launchPrepared(const LaunchState& state, void* workspace, cudaStream
     const PreparedState& prepared = state.prepared;
     const FtcudaGemmDesc& desc    = prepared.desc;
     unsigned char* const base     = reinterpret_cast<unsigned char*>((reinterpret_cast<std::uintptr_t>(workspace) + 255) & ~std::uintptr_t{255});
-    Control* const control        = reinterpret_cast<Control*>(base);
-    cudaError_t error             = cudaMemsetAsync(base, 0, prepared.cleared_bytes, stream);
-    if (error != cudaSuccess) { return error; }
+    std::uint32_t* const decision = reinterpret_cast<std::uint32_t*>(base);
+    std::uint32_t* const verdicts = reinterpret_cast<std::uint32_t*>(base + prepared.verdicts_at);
 
     fp16x3::SplitParams split{};
     split.k        = static_cast<std::uint32_t>(desc.k);
     split.k_blocks = static_cast<std::uint32_t>(ceilDiv(desc.k, kBlockK));
-    split.control  = control;
-    const struct {
-        const float* source;
-        std::int64_t row_stride, k_stride;
-        std::uint64_t rows;
-    } sources[2] = {{desc.a, desc.a_row_stride, desc.a_col_stride, desc.m}, {desc.b, desc.b_col_stride, desc.b_row_stride, desc.n}};
+    split.slabs    = static_cast<std::uint32_t>(ceilDiv(split.k_blocks, kSlabBlocks));
+    describeOperands(desc, split.operand);
     for (int i = 0; i < 2; ++i) {
         fp16x3::SplitOperand& o = split.operand[i];
-        o.source                = sources[i].source;
-        o.row_stride            = sources[i].row_stride;
-        o.k_stride              = sources[i].k_stride;
-        o.rows                  = static_cast<std::uint32_t>(sources[i].rows);
         o.split                 = base + prepared.split_at[i];
-        o.row_max               = reinterpret_cast<std::uint32_t*>(base + prepared.max_at[i]);
-        o.few                   = reinterpret_cast<std::uint32_t*>(base + prepared.few_at[i]);
         o.inverse               = reinterpret_cast<float*>(base + prepared.inverse_at[i]);
-        fp16x3::planSplit(o, split.k);
+        o.pitch                 = prepared.inverse_pitch[i];
+        fp16x3::planSplit(o, split.slabs);
+        o.verdicts = verdicts + (i == 0 ? 0 : split.operand[0].blocks);
     }
-    error = fp16x3::launchSplit(split, stream);
+    cudaError_t error = fp16x3::launchSplit(split, stream);
     if (error != cudaSuccess) { return error; }
 
     CUtensorMap map_a = prepared.map_a, map_b = prepared.map_b;
@@ -564,29 +657,48 @@ cudaError_t launchPrepared(const LaunchState& state, void* workspace, cudaStream
     p.partials         = prepared.splits > 1 ? reinterpret_cast<float*>(base + prepared.partials_at) : nullptr;
     p.inverse_a        = split.operand[0].inverse;
     p.inverse_b        = split.operand[1].inverse;
-    p.control          = control;
+    p.inverse_pitch_a  = prepared.inverse_pitch[0];
+    p.inverse_pitch_b  = prepared.inverse_pitch[1];
+    p.verdicts         = verdicts;
+    p.verdicts_a       = split.operand[0].blocks;
+    p.verdicts_b       = split.operand[1].blocks;
+    p.use_fallback     = decision;
     p.status           = state.device_status;
-    const auto aligned = [](const float* at, std::int64_t row_stride, std::int64_t col_stride) {
-        return col_stride == 1 && row_stride % 4 == 0 && reinterpret_cast<std::uintptr_t>(at) % 16 == 0;
+    const auto aligned = [&](std::uint32_t width, const float* at, std::int64_t row_stride, std::int64_t col_stride) {
+        return desc.n % width == 0 && col_stride == 1 && row_stride % width == 0 && reinterpret_cast<std::uintptr_t>(at) % (4 * width) == 0;
     };
-    p.vector = p.partials != nullptr ? (desc.n % 4 == 0 ? 1U : 0U)
-               : aligned(desc.d, desc.d_row_stride, desc.d_col_stride) && (desc.c == nullptr || aligned(desc.c, desc.c_row_stride, desc.c_col_stride))
-                   ? 1U
-                   : 0U;
+    for (const std::uint32_t width : {8U, 4U}) {
+        const bool fits = p.partials != nullptr ? aligned(width, p.partials, static_cast<std::int64_t>(desc.n), 1)
+                                                : aligned(width, desc.d, desc.d_row_stride, desc.d_col_stride) &&
+                                                      (desc.c == nullptr || aligned(width, desc.c, desc.c_row_stride, desc.c_col_stride));
+        if (fits) {
+            p.vector = width;
+            break;
+        }
+    }
     const std::uint32_t items = p.tiles_m * p.tiles_n * p.splits;
-    tensorGemm3xFp16<<<prepared.grid, kThreads, kSmemBytes, stream>>>(map_a, map_b, p, items);
-    error = cudaGetLastError();
+    cudaLaunchConfig_t config{};
+    config.gridDim          = dim3(prepared.grid, 1, 1);
+    config.blockDim         = dim3(kThreads, 1, 1);
+    config.dynamicSmemBytes = kSmemBytes;
+    config.stream           = stream;
+    cudaLaunchAttribute attribute{};
+    attribute.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs                                         = &attribute;
+    config.numAttrs                                      = 1;
+    error = cudaLaunchKernelEx(&config, tensorGemm3xFp16, map_a, map_b, p, items);
     if (error != cudaSuccess) { return error; }
     countLaunches(1);
     if (prepared.splits > 1) {
-        error = launchSplitKReduce(desc, p.partials, prepared.splits, stream, &control->use_fallback, false);
+        error = launchSplitKReduce(desc, p.partials, prepared.splits, stream, decision, false);
         if (error != cudaSuccess) { return error; }
         countLaunches(1);
     }
     LaunchState fallback = state;
     fallback.kernel      = prepared.fallback_kernel;
-    fallback.run_if      = &control->use_fallback;
-    return launchTensorStaged(fallback, base + prepared.split_at[0], stream, message, capacity);
+    fallback.run_if      = decision;
+    return launchTensorStaged(fallback, base + 256, stream, message, capacity);
 }
 
 }  // namespace ftcuda

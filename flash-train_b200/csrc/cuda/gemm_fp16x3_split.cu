@@ -1,24 +1,28 @@
 // Splits A and B into pairs of FP16 numbers for gemm_fp16x3.cu.
 //
-// Every row of A and every column of B ("row" below, for both) is scaled by a power of two that
-// brings its largest magnitude to [2^14, 2^15), and every scaled element x becomes
+// A "row" below is a row of A or a column of B. K is cut into slabs of 768. In each slab every row of A, and
+// every 16 columns of B together, are scaled by a power of two that brings their largest magnitude there to
+// [2^14, 2^15), and every scaled element x becomes
 //   hi = fp16(x),  lo = fp16((x - hi) * 2^11)      (both to nearest even)
 // so that x = hi + lo / 2^11 to within 2^-24 |x| as long as |x| >= 2^-12, i.e. for every element within
-// 2^26 of its row's largest; below that ("gray" elements) to within 2^-36, which is 2^-50 of the largest.
+// 2^26 of the largest; below that ("gray" elements) to within 2^-36, which is 2^-50 of the largest.
 //
-// When that is enough. An element's error e contributes e * |b| to the result. For gray elements of a row of A
-// the bound is 2^-50 max|a| max|b| each. If at least F_a elements of every row of A, and F_b of every
-// column of B, reach 2^-8 of their row's largest, then any row and column have F_a + F_b - K positions
-// where both do, so sum |a||b| >= (F_a + F_b - K) 2^-16 max|a| max|b|. With F_a + F_b - K >= K / 64 all
-// gray elements of both together add at most 2 K 2^-50 against (K / 64) 2^-16: 2^-27 of sum |a||b| -- below
-// the rounding of an FP32 product. Otherwise, or when a row's largest magnitude is outside
-// [2^-60, 2^60], infinite or NaN, the launch is left to the TF32 kernel, which splits without
-// scaling. No gray element at all needs no such count. The last CTA decides, on the device, for the
-// whole launch.
+// When that is enough. An element's error e contributes e * |b| to the result: for a gray element of A at most
+// 2^-50 M_a M_b, with M the largest magnitude that either scale allows for. If at least F_a elements of every row of A
+// reach 2^-s M_a and F_b of every column of B reach 2^-t M_b, any row and column have F_a + F_b - 768
+// positions where both do, so sum |a||b| over the slab is at least (F_a + F_b - 768) 2^-(s+t) M_a M_b. With
+// s + t = 18 and F_a + F_b - 768 >= 12, all gray elements of both add at most 2 * 768 * 2^-50 against 12 * 2^-18:
+// 2^-25 of sum |a||b|, below the rounding of an FP32 product. The elements are counted for s (and t) of 5, 9 and 13, so
+// that an operand with a few very large elements -- outliers of activations -- is made up for by an even one. No gray
+// element at all needs no count. Otherwise, or when a largest magnitude is outside [2^-100, 2^61), infinite or
+// NaN, the launch is left to the TF32 kernel, which splits without scaling. Every CTA leaves a verdict; the
+// multiplying kernel takes the worst of them all.
 //
-// Both kernels are HBM-bound: the first reads the operands once (4 bytes an element), the second
-// reads them again (from L2 when they fit) and writes as many bytes. At 16384 x 4096 x 14336 (502 MB of operands) 98 + 217 us,
-// 5.1 and 4.6 TB/s.
+// The scales belong to slabs, and not to whole rows, so that one pass is enough: a CTA holds a slab of
+// some rows, takes their largest magnitudes, and converts. HBM-bound: 4 bytes read and 4 written an element.
+// At 4096 x 4096 for each operand (134 MB read, as many written; 41 us at the copy rate) 49 us with both sources along K,
+// 56 with both along their rows. (A pass over the operands for whole rows' maxima and a second one that
+// converted took 31 + 65 us, and 4 us more in launches.)
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -26,22 +30,31 @@
 
 #include "fp16x3.hpp"
 #include "gemm_kernels.hpp"
+#include "ptx.cuh"
 
 namespace ftcuda {
 namespace fp16x3 {
 namespace {
 
-constexpr int kThreads           = 256;
-constexpr std::uint32_t kMaxK    = 2048;  // row_max, source along K: 8 rows x 2048 K values per CTA
-constexpr std::uint32_t kSplitK  = 1024;  // split, source along K: 8 rows x 1024 K values
-constexpr std::uint32_t kTileR   = 128;   // source along its rows: 128 rows x ...
-constexpr std::uint32_t kMaxTall = 128;   // ... 128 K values (row_max)
-constexpr std::uint32_t kSplitTall = 256; // ... 256 K values (split)
+constexpr int kThreads = 512;
+constexpr int kWarps   = kThreads / 32;
+static_assert(kWarps == 2 * kSplitRows / 4 && kSlabBlocks % 2 == 0, "a warp takes four rows, half of the K blocks");
+static_assert(kSplitRowsAlongK == kWarps && kSplitRowsAlongK == kColumnGroup, "a warp takes a row, a CTA a group of columns");
+// A slab of 32 rows, [k][row]: the odd pitch keeps the stores free of bank conflicts and the loads along K within two
+// accesses to a bank.
+constexpr int kTilePitch = static_cast<int>(kSplitRows) + 1;
+constexpr int kTileBytes = static_cast<int>(kSlabK) * kTilePitch * 4;
 
-constexpr std::uint32_t kLowestExponent  = 127 - 60;
+constexpr std::uint32_t kLowestExponent  = 127 - 100;
 constexpr std::uint32_t kHighestExponent = 127 + 60;
 
-__device__ __forceinline__ std::uint32_t magnitude(float value) { return __float_as_uint(value) & 0x7FFFFFFFU; }
+// The larger magnitude; a NaN stays.
+__device__ __forceinline__ float largerMagnitude(float a, float b) {
+    float result;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(result) : "f"(a), "f"(fabsf(b)));
+    return result;
+}
+__device__ __forceinline__ std::uint32_t warpMax(float magnitude) { return __reduce_max_sync(0xFFFFFFFFU, __float_as_uint(magnitude)); }
 
 // Four consecutive K values of a row, zeros beyond the end.
 __device__ __forceinline__ float4 loadAlongK(const SplitOperand& o, const float* row, std::uint32_t k, std::uint32_t depth) {
@@ -55,56 +68,7 @@ __device__ __forceinline__ float4 loadAlongK(const SplitOperand& o, const float*
     return v;
 }
 
-__global__ void __launch_bounds__(kThreads) splitRowMax(const SplitParams p) {
-    const std::uint32_t which = blockIdx.x < p.operand[0].max_blocks ? 0 : 1;
-    const SplitOperand& o     = p.operand[which];
-    const std::uint32_t block = blockIdx.x - (which != 0 ? p.operand[0].max_blocks : 0);
-    const std::uint32_t warp  = threadIdx.x >> 5;
-    const std::uint32_t lane  = threadIdx.x & 31;
-    if (o.along_k != 0) {
-        const std::uint32_t pieces = (p.k + kMaxK - 1) / kMaxK;
-        const std::uint32_t row    = block / pieces * 8 + warp;
-        const std::uint32_t begin  = block % pieces * kMaxK;
-        if (row >= o.rows) { return; }
-        const float* source  = o.source + static_cast<std::int64_t>(row) * o.row_stride;
-        std::uint32_t most   = 0;
-#pragma unroll 8
-        for (std::uint32_t i = 0; i < kMaxK / 128; ++i) {
-            const float4 v = loadAlongK(o, source, begin + i * 128 + lane * 4, p.k);
-            most = max(max(max(most, magnitude(v.x)), max(magnitude(v.y), magnitude(v.z))), magnitude(v.w));
-        }
-        most = __reduce_max_sync(0xFFFFFFFFU, most);
-        if (lane == 0 && most != 0) { atomicMax(o.row_max + row, most); }
-        return;
-    }
-    // Along the rows: 32 consecutive rows per load, a warp takes 16 of the 128 K values.
-    __shared__ std::uint32_t most_of[8][kTileR];
-    const std::uint32_t pieces = (p.k + kMaxTall - 1) / kMaxTall;
-    const std::uint32_t row0   = block / pieces * kTileR;
-    const std::uint32_t begin  = block % pieces * kMaxTall + warp * (kMaxTall / 8);
-    std::uint32_t most[4]      = {0, 0, 0, 0};
-#pragma unroll 4
-    for (std::uint32_t i = 0; i < kMaxTall / 8; ++i) {
-        const std::uint32_t k = begin + i;
-        const float* source   = o.source + static_cast<std::int64_t>(k) * o.k_stride;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const std::uint32_t row = row0 + lane + 32 * j;
-            if (k < p.k && row < o.rows) { most[j] = max(most[j], magnitude(source[static_cast<std::int64_t>(row) * o.row_stride])); }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { most_of[warp][lane + 32 * j] = most[j]; }
-    __syncthreads();
-    if (threadIdx.x < kTileR && row0 + threadIdx.x < o.rows) {
-        std::uint32_t all = 0;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) { all = max(all, most_of[w][threadIdx.x]); }
-        if (all != 0) { atomicMax(o.row_max + row0 + threadIdx.x, all); }
-    }
-}
-
-// What a row's largest magnitude says about its scaling.
+// What a row's largest magnitude (its bit pattern) says about its scaling.
 struct RowScale {
     float scale, inverse;
     bool covered;  // false: the row's magnitudes are out of range (the scale is then 1)
@@ -117,189 +81,283 @@ __device__ __forceinline__ RowScale rowScale(std::uint32_t most) {
     return {__uint_as_float((268 - exponent) << 23), __uint_as_float((exponent - 14) << 23), true};
 }
 
-// hi | lo of one scaled element; counts what the decision needs.
-__device__ __forceinline__ void splitElement(float x, __half& hi, __half& lo, std::uint32_t& few, bool& gray) {
-    hi = __float2half_rn(x);
-    lo = __float2half_rn((x - __half2float(hi)) * 2048.0F);
-    const float size = fabsf(x);
-    few += size < 128.0F ? 1U : 0U;              // 2^-8 of 2^15, the largest a row can hold
-    gray = gray || (size < 0x1p-12F && x != 0.0F);
-}
+// Splits pairs of elements of one row and keeps what the verdict needs: how many reach each threshold (in the scaled
+// numbers, whose largest is below 2^15), and the smallest nonzero magnitude.
+struct PairSplitter {
+    float2 scale;
+    __half2 large[3];                  // counts, in halves: at most 2048 each
+    std::uint32_t least = 0xFFFFFFFFU; // twice the bit pattern of a magnitude, less one
 
-__device__ __forceinline__ std::uint32_t packed(__half a, __half b) {
-    return static_cast<std::uint32_t>(__half_as_ushort(a)) | (static_cast<std::uint32_t>(__half_as_ushort(b)) << 16);
-}
-
-// Called by every thread of the CTA once its part is done. The last CTA of the grid decides.
-__device__ __forceinline__ void finishSplit(const SplitParams& p) {
-    __shared__ std::uint32_t last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) { last = atomicAdd(&p.control->blocks_done, 1U) + 1 == gridDim.x ? 1U : 0U; }
-    __syncthreads();
-    if (last == 0) { return; }
-    __threadfence();
-    const volatile Control* control = p.control;
-    bool fallback                   = control->out_of_range != 0;
-    if (!fallback && control->gray != 0) {
-        // The largest number of small elements in a row, per operand.
-        __shared__ std::uint32_t worst[2];
-        if (threadIdx.x < 2) { worst[threadIdx.x] = 0; }
-        __syncthreads();
-        for (int which = 0; which < 2; ++which) {
-            const SplitOperand& o = p.operand[which];
-            std::uint32_t most    = 0;
-#pragma unroll 8
-            for (std::uint32_t row = threadIdx.x; row < o.rows; row += kThreads) { most = max(most, __ldcg(o.few + row)); }
-            most = __reduce_max_sync(0xFFFFFFFFU, most);
-            if ((threadIdx.x & 31) == 0) { atomicMax(&worst[which], most); }
-        }
-        __syncthreads();
-        // F_a + F_b - K = K - worst_a - worst_b.
-        fallback = static_cast<std::uint64_t>(worst[0]) + worst[1] + p.k / 64 + 1 > p.k;
+    __device__ __forceinline__ explicit PairSplitter(float s) : scale(make_float2(s, s)) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t) { large[t] = __half2half2(__ushort_as_half(0)); }
     }
-    if (threadIdx.x == 0) { p.control->use_fallback = fallback ? 1U : 0U; }
+    __device__ __forceinline__ void split(float a, float b, std::uint32_t& hi, std::uint32_t& lo) {
+        least = min(least, min(__float_as_uint(a) * 2U - 1U, __float_as_uint(b) * 2U - 1U));  // zero: the largest number
+        const float2 x   = multiply2(make_float2(a, b), scale);
+        const __half2 h  = __float22half2_rn(x);
+        const float2 up  = multiply2(x, make_float2(2048.0F, 2048.0F));
+        const float2 low = multiplyAdd2(__half22float2(h), make_float2(-2048.0F, -2048.0F), up);  // exact
+        const __half2 l  = __float22half2_rn(low);
+        const __half2 m  = __habs2(h);
+        large[0] = __hadd2(large[0], __hge2(m, __float2half2_rn(0x1p10F)));
+        large[1] = __hadd2(large[1], __hge2(m, __float2half2_rn(0x1p6F)));
+        large[2] = __hadd2(large[2], __hge2(m, __float2half2_rn(0x1p2F)));
+        hi       = *reinterpret_cast<const std::uint32_t*>(&h);
+        lo       = *reinterpret_cast<const std::uint32_t*>(&l);
+    }
+    // The three counts, ten bits each (a slab of one row has at most 768).
+    __device__ __forceinline__ std::uint32_t largeElements() const {
+        std::uint32_t all = 0;
+#pragma unroll
+        for (int t = 0; t < 3; ++t) { all |= static_cast<std::uint32_t>(__low2float(large[t]) + __high2float(large[t])) << (10 * t); }
+        return all;
+    }
+    __device__ __forceinline__ bool sawGray() const {
+        return least != 0xFFFFFFFFU && __uint_as_float((least + 1U) / 2U) * scale.x < 0x1p-12F;
+    }
+};
+
+// For each threshold the larger number of small elements, of `length`, given counts of large ones.
+__device__ __forceinline__ void worstCounts(std::uint32_t (&worst)[3], std::uint32_t large, std::uint32_t length) {
+#pragma unroll
+    for (int t = 0; t < 3; ++t) { worst[t] = max(worst[t], length - (large >> (10 * t) & 0x3FFU)); }
 }
 
-__global__ void __launch_bounds__(kThreads) splitOperands(const SplitParams p) {
-    const std::uint32_t which = blockIdx.x < p.operand[0].split_blocks ? 0 : 1;
+__global__ void __launch_bounds__(kThreads, 2) splitOperands(const SplitParams p) {
+    extern __shared__ float tile[];
+    __shared__ std::uint32_t most_of[kWarps][kSplitRows];
+    __shared__ std::uint32_t large_of[kSplitRows];
+    __shared__ float scale_of[kSplitRows];
+    __shared__ std::uint32_t worst_of[kWarps][3], flags_of[kWarps];
+    const std::uint32_t which = blockIdx.x < p.operand[0].blocks ? 0 : 1;
     const SplitOperand& o     = p.operand[which];
-    const std::uint32_t block = blockIdx.x - (which != 0 ? p.operand[0].split_blocks : 0);
+    const std::uint32_t block = blockIdx.x - (which != 0 ? p.operand[0].blocks : 0);
     const std::uint32_t warp  = threadIdx.x >> 5;
     const std::uint32_t lane  = threadIdx.x & 31;
     const std::uint64_t pitch = p.k_blocks * kBlockBytes;
     bool gray                 = false;
     bool covered              = true;
+    std::uint32_t worst[3]    = {0, 0, 0};  // small elements of the worst row this thread knows
+    gridDependencyWait();
+    gridDependencyLaunchDependents();
+    std::uint32_t slab, row0;
+    if (o.along_k != 0) {  // neighbouring CTAs take neighbouring pieces of memory
+        slab = block % p.slabs;
+        row0 = block / p.slabs * kSplitRowsAlongK;
+    } else {
+        const std::uint32_t row_blocks = (o.rows + kSplitRows - 1) / kSplitRows;
+        slab = block / row_blocks;
+        row0 = block % row_blocks * kSplitRows;
+    }
+    const std::uint32_t begin  = slab * kSlabK;
+    const std::uint32_t depth  = min(p.k, begin + kSlabK);
+    const std::uint32_t length = depth - begin;
+    const std::uint32_t k_end  = min(p.k_blocks * kBlockK, begin + kSlabK);
     if (o.along_k != 0) {
-        const std::uint32_t pieces = (p.k + kSplitK - 1) / kSplitK;
-        const std::uint32_t row    = block / pieces * 8 + warp;
-        const std::uint32_t begin  = block % pieces * kSplitK;
+        // A warp takes a row, 128 K values per load.
+        const std::uint32_t row = row0 + warp;
+        const float* source     = o.source + static_cast<std::int64_t>(row) * o.row_stride;
+        float4 v[kSlabK / 128];
+#pragma unroll
+        for (std::uint32_t i = 0; i < kSlabK / 128; ++i) {
+            v[i] = row < o.rows ? loadAlongK(o, source, begin + i * 128 + lane * 4, depth) : make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+        }
+        float magnitude = 0.0F;
+#pragma unroll
+        for (std::uint32_t i = 0; i < kSlabK / 128; ++i) {
+            magnitude = largerMagnitude(largerMagnitude(magnitude, v[i].x), v[i].y);
+            magnitude = largerMagnitude(largerMagnitude(magnitude, v[i].z), v[i].w);
+        }
+        const std::uint32_t most = warpMax(magnitude);
+        std::uint32_t of_group   = most;
+        if (o.grouped != 0) {
+            if (lane == 0) { large_of[warp] = most; }
+            __syncthreads();
+            of_group = __reduce_max_sync(0xFFFFFFFFU, large_of[lane % kWarps]);
+        }
+        const RowScale scaling = rowScale(of_group);
+        covered                = scaling.covered;
         if (row < o.rows) {
-            const RowScale scaling = rowScale(o.row_max[row]);
-            const bool zero_row    = o.row_max[row] == 0;
-            covered                = scaling.covered;
-            const float* source    = o.source + static_cast<std::int64_t>(row) * o.row_stride;
-            unsigned char* target  = o.split + row * pitch;
-            std::uint32_t few      = 0;
-            const std::uint32_t k_end = p.k_blocks * kBlockK;
-            float4 v[kSplitK / 128];
+            unsigned char* target = o.split + row * pitch + begin / kBlockK * kBlockBytes + lane / 16 * kBlockBytes + lane % 16 * 8;
+            PairSplitter splitter(scaling.scale);
 #pragma unroll
-            for (std::uint32_t i = 0; i < kSplitK / 128; ++i) { v[i] = loadAlongK(o, source, begin + i * 128 + lane * 4, p.k); }
-#pragma unroll
-            for (std::uint32_t i = 0; i < kSplitK / 128; ++i) {
-                const std::uint32_t k = begin + i * 128 + lane * 4;
-                if (k >= k_end) { continue; }
-                __half hi[4], lo[4];
-                splitElement(v[i].x * scaling.scale, hi[0], lo[0], few, gray);
-                splitElement(v[i].y * scaling.scale, hi[1], lo[1], few, gray);
-                splitElement(v[i].z * scaling.scale, hi[2], lo[2], few, gray);
-                splitElement(v[i].w * scaling.scale, hi[3], lo[3], few, gray);
-                // The zeros that fill up the last K block are not elements.
-                if (k + 4 > p.k) { few -= k >= p.k ? 4U : k + 4 - p.k; }
-                unsigned char* at = target + k / kBlockK * kBlockBytes + k % kBlockK * 2;
-                *reinterpret_cast<uint2*>(at)               = make_uint2(packed(hi[0], hi[1]), packed(hi[2], hi[3]));
-                *reinterpret_cast<uint2*>(at + 2 * kBlockK) = make_uint2(packed(lo[0], lo[1]), packed(lo[2], lo[3]));
+            for (std::uint32_t i = 0; i < kSlabK / 128; ++i) {
+                uint2 hi, lo;
+                splitter.split(v[i].x, v[i].y, hi.x, lo.x);
+                splitter.split(v[i].z, v[i].w, hi.y, lo.y);
+                if (begin + i * 128 + lane * 4 < k_end) {
+                    *reinterpret_cast<uint2*>(target + i * 2 * kBlockBytes)               = hi;
+                    *reinterpret_cast<uint2*>(target + i * 2 * kBlockBytes + 2 * kBlockK) = lo;
+                }
             }
-            few = __reduce_add_sync(0xFFFFFFFFU, few);
-            if (lane == 0) {
-                if (few != 0 && !zero_row) { atomicAdd(o.few + row, few); }
-                if (begin == 0) { o.inverse[row] = scaling.inverse; }
-            }
+            gray                      = splitter.sawGray();
+            const std::uint32_t large = __reduce_add_sync(0xFFFFFFFFU, splitter.largeElements());
+            if (most != 0) { worstCounts(worst, large, length); }
+            if (lane == 0) { o.inverse[slab * o.pitch + (o.grouped != 0 ? row / kColumnGroup : row)] = scaling.inverse; }
         }
     } else {
-        // The tile is turned in shared memory: read along the rows, written along K. An odd pitch keeps
-        // both sides within two accesses to a bank.
-        __shared__ float tile[kBlockK][kTileR + 1];
-        const std::uint32_t pieces = (p.k + kSplitTall - 1) / kSplitTall;
-        const std::uint32_t row0   = block / pieces * kTileR;
-        const std::uint32_t begin  = block % pieces * kSplitTall;
-        const std::uint32_t eighth = lane & 7;  // this thread's 8 K values of a block
-        std::uint32_t few[4]       = {0, 0, 0, 0};
-        RowScale scaling[4];
-        bool zero_row[4];
+        // The slab is turned in shared memory: read along the rows, written along K.
+        if (threadIdx.x < kSplitRows) { large_of[threadIdx.x] = 0; }
+        if (o.vector != 0) {
+            // 16-byte loads: a warp takes 4 K values of all 32 rows.
+            const std::uint32_t at_row = lane % 8 * 4;
+            const std::uint32_t row    = row0 + at_row;
+            const bool whole           = row + 4 <= o.rows;
+            float most[4]              = {0.0F, 0.0F, 0.0F, 0.0F};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const std::uint32_t row  = row0 + warp * 16 + j * 4 + lane / 8;
-            const std::uint32_t most = row < o.rows ? o.row_max[row] : 0;
-            scaling[j]               = rowScale(most);
-            zero_row[j]              = most == 0;
-            covered                  = covered && scaling[j].covered;
-            if (begin == 0 && eighth == 0 && row < o.rows) { o.inverse[row] = scaling[j].inverse; }
-        }
-        for (std::uint32_t k0 = begin; k0 < begin + kSplitTall && k0 < p.k; k0 += kBlockK) {
-            float v[8][4];
+            for (int batch = 0; batch < 2; ++batch) {
+                float4 v[6];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const std::uint32_t k = k0 + warp * 8 + i;
-                const float* source   = o.source + static_cast<std::int64_t>(k) * o.k_stride;
+                for (int i = 0; i < 6; ++i) {
+                    const std::uint32_t k = begin + (batch * 6 + i) * 64 + warp * 4 + lane / 8;
+                    const float* source   = o.source + static_cast<std::int64_t>(k) * o.k_stride + row;
+                    v[i]                  = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+                    if (k < depth) {
+                        if (whole) {
+                            v[i] = *reinterpret_cast<const float4*>(source);
+                        } else {
+                            if (row < o.rows) { v[i].x = source[0]; }
+                            if (row + 1 < o.rows) { v[i].y = source[1]; }
+                            if (row + 2 < o.rows) { v[i].z = source[2]; }
+                        }
+                    }
+                }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const std::uint32_t row = row0 + lane + 32 * j;
-                    v[i][j] = k < p.k && row < o.rows ? source[static_cast<std::int64_t>(row) * o.row_stride] : 0.0F;
+                for (int i = 0; i < 6; ++i) {
+                    float* to = tile + ((batch * 6 + i) * 64 + warp * 4 + lane / 8) * kTilePitch + at_row;
+                    to[0] = v[i].x, to[1] = v[i].y, to[2] = v[i].z, to[3] = v[i].w;
+                    most[0] = largerMagnitude(most[0], v[i].x);
+                    most[1] = largerMagnitude(most[1], v[i].y);
+                    most[2] = largerMagnitude(most[2], v[i].z);
+                    most[3] = largerMagnitude(most[3], v[i].w);
                 }
             }
-            __syncthreads();  // the previous block's tile has been read
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) { tile[warp * 8 + i][lane + 32 * j] = v[i][j]; }
-            }
-            __syncthreads();
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const std::uint32_t in_tile = warp * 16 + j * 4 + lane / 8;
-                const std::uint32_t row     = row0 + in_tile;
-                __half hi[8], lo[8];
-                std::uint32_t small = 0;
+                std::uint32_t bits = __float_as_uint(most[j]);
+                bits = max(bits, __shfl_xor_sync(0xFFFFFFFFU, bits, 8));
+                bits = max(bits, __shfl_xor_sync(0xFFFFFFFFU, bits, 16));
+                if (lane < 8) { most_of[warp][at_row + j] = bits; }
+            }
+        } else {
+            const std::uint32_t row = row0 + lane;
+            float most              = 0.0F;
+#pragma unroll 1
+            for (int batch = 0; batch < 3; ++batch) {
+                float v[16];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    splitElement(tile[eighth * 8 + i][in_tile] * scaling[j].scale, hi[i], lo[i], small, gray);
+                for (int i = 0; i < 16; ++i) {
+                    const std::uint32_t k = begin + (batch * 16 + i) * 16 + warp;
+                    v[i] = k < depth && row < o.rows
+                               ? o.source[static_cast<std::int64_t>(k) * o.k_stride + static_cast<std::int64_t>(row) * o.row_stride]
+                               : 0.0F;
                 }
-                const std::uint32_t k = k0 + eighth * 8;
-                if (k + 8 > p.k) { small -= k >= p.k ? 8U : k + 8 - p.k; }
-                few[j] += small;
-                if (row < o.rows) {
-                    unsigned char* at = o.split + row * pitch + k0 / kBlockK * kBlockBytes + eighth * 16;
-                    *reinterpret_cast<uint4*>(at) = make_uint4(packed(hi[0], hi[1]), packed(hi[2], hi[3]), packed(hi[4], hi[5]), packed(hi[6], hi[7]));
-                    *reinterpret_cast<uint4*>(at + 2 * kBlockK) =
-                        make_uint4(packed(lo[0], lo[1]), packed(lo[2], lo[3]), packed(lo[4], lo[5]), packed(lo[6], lo[7]));
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    tile[((batch * 16 + i) * 16 + warp) * kTilePitch + lane] = v[i];
+                    most = largerMagnitude(most, v[i]);
                 }
             }
+            most_of[warp][lane] = __float_as_uint(most);
         }
+        __syncthreads();
+        std::uint32_t most = 0;
+        if (threadIdx.x < kSplitRows) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const std::uint32_t row = row0 + warp * 16 + j * 4 + lane / 8;
-            std::uint32_t all       = few[j];
-            all += __shfl_xor_sync(0xFFFFFFFFU, all, 1);
-            all += __shfl_xor_sync(0xFFFFFFFFU, all, 2);
-            all += __shfl_xor_sync(0xFFFFFFFFU, all, 4);
-            if (eighth == 0 && row < o.rows && all != 0 && !zero_row[j]) { atomicAdd(o.few + row, all); }
+            for (int w = 0; w < kWarps; ++w) { most = max(most, most_of[w][threadIdx.x]); }
+            std::uint32_t of_group = most;
+            if (o.grouped != 0) {
+                of_group = max(of_group, __shfl_xor_sync(0xFFFFFFFFU, of_group, 1));
+                of_group = max(of_group, __shfl_xor_sync(0xFFFFFFFFU, of_group, 2));
+                of_group = max(of_group, __shfl_xor_sync(0xFFFFFFFFU, of_group, 4));
+                of_group = max(of_group, __shfl_xor_sync(0xFFFFFFFFU, of_group, 8));
+            }
+            const RowScale scaling  = rowScale(of_group);
+            const std::uint32_t row = row0 + threadIdx.x;
+            covered                 = scaling.covered;
+            scale_of[threadIdx.x]   = scaling.scale;
+            if (row < o.rows) { o.inverse[slab * o.pitch + (o.grouped != 0 ? row / kColumnGroup : row)] = scaling.inverse; }
         }
+        __syncthreads();
+        // A warp takes four rows, half of the K blocks; a thread 8 K values of each block.
+        constexpr std::uint32_t kGroups = kSplitRows / 4;
+        const std::uint32_t at_row      = warp % kGroups * 4 + lane / 8;
+        const std::uint32_t first       = warp / kGroups * (kSlabBlocks / 2);
+        const bool inside               = row0 + at_row < o.rows;
+        unsigned char* at = o.split + (row0 + at_row) * pitch + (begin / kBlockK + first) * kBlockBytes + lane % 8 * 16;
+        const float* from = tile + (first * kBlockK + lane % 8 * 8) * kTilePitch + at_row;
+        PairSplitter splitter(scale_of[at_row]);
+#pragma unroll 2
+        for (std::uint32_t i = 0; i < kSlabBlocks / 2; ++i, at += kBlockBytes, from += kBlockK * kTilePitch) {
+            if (begin + (first + i) * kBlockK >= k_end) { break; }
+            uint4 hi, lo;
+            splitter.split(from[0], from[kTilePitch], hi.x, lo.x);
+            splitter.split(from[2 * kTilePitch], from[3 * kTilePitch], hi.y, lo.y);
+            splitter.split(from[4 * kTilePitch], from[5 * kTilePitch], hi.z, lo.z);
+            splitter.split(from[6 * kTilePitch], from[7 * kTilePitch], hi.w, lo.w);
+            if (inside) {
+                *reinterpret_cast<uint4*>(at)               = hi;
+                *reinterpret_cast<uint4*>(at + 2 * kBlockK) = lo;
+            }
+        }
+        gray                = splitter.sawGray();
+        std::uint32_t large = splitter.largeElements();
+        large += __shfl_xor_sync(0xFFFFFFFFU, large, 1);
+        large += __shfl_xor_sync(0xFFFFFFFFU, large, 2);
+        large += __shfl_xor_sync(0xFFFFFFFFU, large, 4);
+        if (lane % 8 == 0) { atomicAdd(&large_of[at_row], large); }
+        __syncthreads();
+        if (threadIdx.x < kSplitRows && most != 0) { worstCounts(worst, large_of[threadIdx.x], length); }
     }
-    if (__any_sync(0xFFFFFFFFU, gray) && lane == 0) { p.control->gray = 1; }
-    if (!__all_sync(0xFFFFFFFFU, covered) && lane == 0) { p.control->out_of_range = 1; }
-    finishSplit(p);
+    const bool any_gray = __any_sync(0xFFFFFFFFU, gray), all_covered = __all_sync(0xFFFFFFFFU, covered);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) { worst[t] = __reduce_max_sync(0xFFFFFFFFU, worst[t]); }
+    if (lane == 0) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t) { worst_of[warp][t] = (worst[t] * 1023 + length - 1) / length; }
+        flags_of[warp] = (any_gray ? kVerdictGray : 0U) | (all_covered ? 0U : kVerdictOutOfRange);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        std::uint32_t few[3] = {0, 0, 0}, verdict = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            verdict |= flags_of[w];
+#pragma unroll
+            for (int t = 0; t < 3; ++t) { few[t] = max(few[t], worst_of[w][t]); }
+        }
+        o.verdicts[block] = verdict | few[0] | few[1] << 10 | few[2] << 20;
+    }
 }
 
 }  // namespace
 
-void planSplit(SplitOperand& o, std::uint32_t k) {
+void planSplit(SplitOperand& o, std::uint32_t slabs) {
     const auto size = [](std::int64_t stride) { return stride < 0 ? -stride : stride; };
     o.along_k       = size(o.k_stride) <= size(o.row_stride) ? 1U : 0U;
-    o.vector        = o.k_stride == 1 && o.row_stride % 4 == 0 && reinterpret_cast<std::uintptr_t>(o.source) % 16 == 0 ? 1U : 0U;
-    const std::uint64_t rows8 = ceilDiv(o.rows, 8), tiles = ceilDiv(o.rows, kTileR);
-    o.max_blocks   = static_cast<std::uint32_t>(o.along_k != 0 ? rows8 * ceilDiv(k, kMaxK) : tiles * ceilDiv(k, kMaxTall));
-    o.split_blocks = static_cast<std::uint32_t>(o.along_k != 0 ? rows8 * ceilDiv(k, kSplitK) : tiles * ceilDiv(k, kSplitTall));
+    const std::int64_t fast = o.along_k != 0 ? o.k_stride : o.row_stride, slow = o.along_k != 0 ? o.row_stride : o.k_stride;
+    o.vector = fast == 1 && slow % 4 == 0 && reinterpret_cast<std::uintptr_t>(o.source) % 16 == 0 ? 1U : 0U;
+    o.blocks = static_cast<std::uint32_t>(ceilDiv(o.rows, o.along_k != 0 ? kSplitRowsAlongK : kSplitRows) * slabs);
+}
+
+cudaError_t configureSplit() {
+    return cudaFuncSetAttribute(splitOperands, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileBytes);
 }
 
 cudaError_t launchSplit(const SplitParams& p, cudaStream_t stream) {
-    splitRowMax<<<p.operand[0].max_blocks + p.operand[1].max_blocks, kThreads, 0, stream>>>(p);
-    cudaError_t error = cudaGetLastError();
-    if (error != cudaSuccess) { return error; }
-    splitOperands<<<p.operand[0].split_blocks + p.operand[1].split_blocks, kThreads, 0, stream>>>(p);
-    error = cudaGetLastError();
-    countLaunches(2);
-    return error;
+    cudaLaunchConfig_t config{};
+    config.gridDim          = dim3(p.operand[0].blocks + p.operand[1].blocks, 1, 1);
+    config.blockDim         = dim3(kThreads, 1, 1);
+    config.dynamicSmemBytes = p.operand[0].along_k != 0 && p.operand[1].along_k != 0 ? 0 : kTileBytes;
+    config.stream           = stream;
+    cudaLaunchAttribute attribute{};
+    attribute.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs                                         = &attribute;
+    config.numAttrs                                      = 1;
+    countLaunches(1);
+    return cudaLaunchKernelEx(&config, splitOperands, p);
 }
 
 }  // namespace fp16x3

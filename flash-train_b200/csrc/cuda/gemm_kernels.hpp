@@ -46,8 +46,7 @@ struct PreparedState {
     std::int32_t fallback_kernel;  // 0 is never a fallback: nonzero marks a prepared launch
     std::uint32_t tile_n, splits, blocks_per_split, chunk_blocks;
     std::uint32_t grid;
-    std::uint64_t cleared_bytes;                  // head of the workspace cleared before the launch
-    std::uint64_t max_at[2], few_at[2], inverse_at[2], split_at[2], partials_at;
+    std::uint64_t verdicts_at, inverse_at[2], inverse_pitch[2], split_at[2], partials_at;  // byte offsets; pitch in elements
 };
 
 // What ftcuda_gemm_configure stores inside an FtcudaGemmLaunch.

@@ -145,7 +145,7 @@ tensorGemm3xTf32(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                  const TensorParams p, const std::uint32_t num_items) {
     extern __shared__ unsigned char smem_raw[];
     if (p.run_if != nullptr) {
-        gridDependencyWait();  // the cluster form may start early
+        gridDependencyWait();  // launched early
         if (*p.run_if == 0) { return; }
     }
     const std::uint32_t align_offset = (1024 - (smemAddress(smem_raw) & 1023)) & 1023;
@@ -820,8 +820,23 @@ cudaError_t launchTensor(const LaunchState& state, void* workspace, cudaStream_t
         return error;
     }
     const std::uint32_t items = p.tiles_m * p.tiles_n * p.splits;
-    tensorGemm3xTf32<false><<<state.grid_x, state.block, state.smem_bytes, stream>>>(state.map_a, state.map_b, p, items);
-    error = cudaGetLastError();
+    if (state.run_if != nullptr) {
+        // As a fallback it mostly leaves at once; its launch overlaps the tail of the kernel it waits for.
+        cudaLaunchConfig_t config{};
+        config.gridDim          = dim3(state.grid_x, 1, 1);
+        config.blockDim         = dim3(state.block, 1, 1);
+        config.dynamicSmemBytes = state.smem_bytes;
+        config.stream           = stream;
+        cudaLaunchAttribute attribute{};
+        attribute.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attribute.val.programmaticStreamSerializationAllowed = 1;
+        config.attrs                                         = &attribute;
+        config.numAttrs                                      = 1;
+        error = cudaLaunchKernelEx(&config, tensorGemm3xTf32<false>, state.map_a, state.map_b, p, items);
+    } else {
+        tensorGemm3xTf32<false><<<state.grid_x, state.block, state.smem_bytes, stream>>>(state.map_a, state.map_b, p, items);
+        error = cudaGetLastError();
+    }
     std::uint64_t launches = 1;
     if (error == cudaSuccess && state.splits > 1) {
         error = launchSplitKReduce(desc, static_cast<const float*>(workspace), state.splits, stream, state.run_if);

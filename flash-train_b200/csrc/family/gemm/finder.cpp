@@ -10,12 +10,17 @@ std::uint64_t ceilDiv(std::uint64_t x, std::uint64_t y) { return (x + y - 1) / y
 
 }  // namespace
 
-// The split reads A and B twice and writes them once, about 35 us of launches and memory passes before the first
-// MMA; the multiplication then takes half the time. Measured (TF32 form / prepared form, microseconds):
-// 2048^3 114 / 98, 4096 x 4096 x 2048 362 / 270, 4096^3 688 / 471, 16384 x 4096 x 14336 8810 / 4520; but
-// 1024^3 25 / 50, 2048 x 8192 x 1024 172 / 194, 1024 x 8192 x 2048 168 / 194.
+// The split passes over (m + n) k elements, the multiplication saves half of the tensor time of m n k, so what counts is
+// m n / (m + n). Measured (better TF32 form / prepared form, microseconds): from 600 on the prepared form is ahead as soon as
+// there is enough work (2048 x 512 x 1024 37 / 29, 1024 x 16384 x 2048 316 / 293, 2048^3 115 / 63, 4096^3 710 / 412,
+// 8192 x 4096 x 8192 2779 / 1438); at 455 and 512 only with a medium K (1024 x 4096 x 1024 59 / 51, 512 x 2048 x 4096 65 / 50,
+// but 1024^3 26 / 27, 512 x 16384 x 4096 326 / 356); below that hardly ever (512 x 4096 x 2048 51 / 60,
+// 256 x 4096 x 4096 50 / 75). A K under 512 was not measured.
 bool preparedFormPays(const GemmShape& shape) noexcept {
-    return shape.m >= 2048 && shape.n >= 2048 && shape.k >= 2048;
+    if (shape.k < 512 || shape.m < 512 || shape.n < 512) { return false; }
+    const double m = static_cast<double>(shape.m), n = static_cast<double>(shape.n), products = m * n * static_cast<double>(shape.k);
+    const double reuse = m * n / (m + n);
+    return reuse >= 600.0 ? products >= 1e9 : reuse >= 450.0 && products >= 1.5e9 && products <= 6e9;
 }
 
 // Regime map on B200 (148 SMs; the count is queried, not assumed). The
