@@ -8,11 +8,14 @@
 //                               output tiles of all groups (gemm_tf32x3.cu, grouped form). The
 //                               per-group table (TMA descriptors, output views) travels in the
 //                               workspace.
+//   FTCUDA_GROUPED_GEMM_FP16X3  the large groups through the prepared form (gemm_fp16x3.cu), one launch sequence
+//                               each, the others as above.
 #include <cuda_runtime_api.h>
 
 #include <new>
 
 #include "gemm_kernels.hpp"
+#include "large_group.hpp"
 
 using ftcuda::fail;
 using ftcuda::GroupedLaunchState;
@@ -23,6 +26,8 @@ struct FtcudaGroupedGemmLaunch {
 
 namespace {
 
+bool preparedGroup(const FtcudaGemmDesc& desc) { return ftcuda::largeGroup(desc) && ftcuda::supportsPrepared(desc) == nullptr; }
+
 const char* supportsGrouped(int kernel, const FtcudaGemmDesc* groups, std::uint32_t count) {
     switch (kernel) {
         case FTCUDA_GROUPED_GEMM_EXACT:
@@ -32,6 +37,11 @@ const char* supportsGrouped(int kernel, const FtcudaGemmDesc* groups, std::uint3
             }
             return nullptr;
         case FTCUDA_GROUPED_GEMM_TF32X3: return ftcuda::supportsTensorGrouped(groups, count);
+        case FTCUDA_GROUPED_GEMM_FP16X3:
+            for (std::uint32_t g = 0; g < count; ++g) {
+                if (preparedGroup(groups[g])) { return ftcuda::supportsTensorGrouped(groups, count); }
+            }
+            return "no group is large enough for the prepared form";
         default: return "unknown grouped kernel family";
     }
 }
@@ -70,6 +80,26 @@ extern "C" int ftcuda_grouped_gemm_configure(int kernel, const FtcudaGemmDesc* g
                     state.host_status = one.host_status;
                 }
             }
+        } else if (kernel == FTCUDA_GROUPED_GEMM_FP16X3) {
+            std::vector<FtcudaGemmDesc> others;
+            std::uint64_t prepared_bytes = 0;
+            for (std::uint32_t g = 0; g < num_groups && status == 0; ++g) {
+                if (!preparedGroup(groups[g])) {
+                    others.push_back(groups[g]);
+                    continue;
+                }
+                FtcudaGemmLaunch one;
+                status = ftcuda_gemm_configure(FTCUDA_GEMM_FP16X3, &groups[g], &one, message, message_capacity);
+                if (status != 0) { break; }
+                const std::uint64_t bytes = ftcuda_gemm_workspace_bytes(&one);
+                prepared_bytes            = bytes > prepared_bytes ? bytes : prepared_bytes;
+                state.prepared.push_back(one);
+            }
+            if (status == 0) {
+                status = ftcuda::configureTensorGrouped(state, others.data(), static_cast<std::uint32_t>(others.size()), message, message_capacity);
+                state.prepared_at = (state.workspace_bytes + 255) / 256 * 256;
+                state.workspace_bytes = state.prepared_at + prepared_bytes;
+            }
         } else {
             status = ftcuda::configureTensorGrouped(state, groups, num_groups, message, message_capacity);
         }
@@ -105,6 +135,13 @@ extern "C" int ftcuda_grouped_gemm_launch(const FtcudaGroupedGemmLaunch* launch,
         }
     } else {
         error = ftcuda::launchTensorGrouped(state, workspace, cuda_stream);
+        for (const FtcudaGemmLaunch& one : state.prepared) {
+            if (error != cudaSuccess) { break; }
+            if (const int status = ftcuda_gemm_launch(&one, static_cast<unsigned char*>(workspace) + state.prepared_at,
+                                                      workspace_bytes - state.prepared_at, stream, message, message_capacity)) {
+                return status;
+            }
+        }
     }
     if (error != cudaSuccess) { return fail(message, message_capacity, 1, "%s", cudaGetErrorString(error)); }
     return 0;

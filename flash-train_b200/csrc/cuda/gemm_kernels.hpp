@@ -187,6 +187,9 @@ struct GroupedLaunchState {
     std::uint64_t workspace_bytes = 0;
     int* device_status            = nullptr;
     volatile int* host_status     = nullptr;
+    // FTCUDA_GROUPED_GEMM_FP16X3: the large groups' launches; their common workspace lies behind the table.
+    std::vector<FtcudaGemmLaunch> prepared;
+    std::uint64_t prepared_at = 0;
 };
 
 // The persistent tensor-core kernel over the tiles of all groups (gemm_tf32x3.cu).

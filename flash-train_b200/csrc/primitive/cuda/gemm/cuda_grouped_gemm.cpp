@@ -1,6 +1,9 @@
 #include "primitive/cuda/gemm/cuda_grouped_gemm.hpp"
 
+#include <algorithm>
 #include <cstdint>
+
+#include "cuda/large_group.hpp"
 
 namespace ftrain {
 namespace {
@@ -98,24 +101,42 @@ Result CudaGroupedGemm::isApplicable(const GroupedGemmProblem& problem, const Co
 
 void CudaGroupedGemm::configure(const GroupedGemmProblem& problem) {
     launch_.reset();
+    prepared_.reset();
     workspace_bytes_ = 0;
     if (problem.hasEmptyOutput()) { return; }
     const std::vector<FtcudaGemmDesc> descs = makeCudaGroupedDescs(problem, getCurrentDeviceId(), true);
     char reason[256];
     reason[0]                      = '\0';
-    FtcudaGroupedGemmLaunch* made = nullptr;
-    if (ftcuda_grouped_gemm_configure(kernel_, descs.data(), static_cast<std::uint32_t>(descs.size()), &made, reason, sizeof reason) != 0) {
-        throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "%s: configuring the launch failed: %s", getName(), reason);
+    const auto count = static_cast<std::uint32_t>(descs.size());
+    const auto make  = [&](int kernel) {
+        FtcudaGroupedGemmLaunch* made = nullptr;
+        if (ftcuda_grouped_gemm_configure(kernel, descs.data(), count, &made, reason, sizeof reason) != 0) {
+            throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "%s: configuring the launch failed: %s", getName(), reason);
+        }
+        return std::shared_ptr<FtcudaGroupedGemmLaunch>(made, [](FtcudaGroupedGemmLaunch* launch) { ftcuda_grouped_gemm_destroy(launch); });
+    };
+    launch_          = make(kernel_);
+    workspace_bytes_ = ftcuda_grouped_gemm_workspace_bytes(launch_.get());
+    if (kernel_ == FTCUDA_GROUPED_GEMM_TF32X3 && std::any_of(descs.begin(), descs.end(), ftcuda::largeGroup) &&
+        ftcuda_grouped_gemm_supports(FTCUDA_GROUPED_GEMM_FP16X3, descs.data(), count, reason, sizeof reason) == 0) {
+        prepared_       = make(FTCUDA_GROUPED_GEMM_FP16X3);
+        prepared_bytes_ = ftcuda_grouped_gemm_workspace_bytes(prepared_.get());
     }
-    launch_.reset(made, [](FtcudaGroupedGemmLaunch* launch) { ftcuda_grouped_gemm_destroy(launch); });
-    workspace_bytes_ = ftcuda_grouped_gemm_workspace_bytes(made);
+}
+
+std::unique_ptr<PrimitiveBase> CudaGroupedGemm::cloneForMinimumWorkspace() const {
+    if (prepared_ == nullptr) { return nullptr; }
+    auto lean = std::make_unique<CudaGroupedGemm>(*this);
+    lean->prepared_.reset();
+    return lean;
 }
 
 void CudaGroupedGemm::executeImpl(const Resources& resources) {
     if (launch_ == nullptr) { return; }
     char reason[256];
     reason[0] = '\0';
-    if (ftcuda_grouped_gemm_launch(launch_.get(), resources.getWorkspace(), resources.getWorkspaceBytes(), resources.getStream(), reason,
+    const bool prepared = prepared_ != nullptr && resources.getWorkspace() != nullptr && resources.getWorkspaceBytes() >= prepared_bytes_;
+    if (ftcuda_grouped_gemm_launch(prepared ? prepared_.get() : launch_.get(), resources.getWorkspace(), resources.getWorkspaceBytes(), resources.getStream(), reason,
                                    sizeof reason) != 0) {
         throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "grouped FP32 GEMM kernel launch failed: %s", reason);
     }

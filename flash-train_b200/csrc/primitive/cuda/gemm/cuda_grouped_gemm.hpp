@@ -31,7 +31,11 @@ class CudaGroupedGemm final : public Primitive<GroupedGemmProblem> {
     // A clone shares the configured launch (immutable once made); configuring the clone replaces it.
     std::unique_ptr<PrimitiveBase> clone() const override { return std::make_unique<CudaGroupedGemm>(*this); }
     Result isApplicable(const GroupedGemmProblem& problem, const Constraints& constraints) const override;
-    std::uint64_t getRequiredWorkspaceBytes() const noexcept override { return workspace_bytes_; }
+    std::uint64_t getRequiredWorkspaceBytes() const noexcept override {
+        return prepared_ != nullptr ? prepared_bytes_ : workspace_bytes_;
+    }
+    std::uint64_t getMinimumWorkspaceBytes() const noexcept override { return workspace_bytes_; }
+    std::unique_ptr<PrimitiveBase> cloneForMinimumWorkspace() const override;
     void configure(const GroupedGemmProblem& problem) override;
 
   private:
@@ -40,6 +44,9 @@ class CudaGroupedGemm final : public Primitive<GroupedGemmProblem> {
     int kernel_;
     std::uint64_t workspace_bytes_{0};
     std::shared_ptr<FtcudaGroupedGemmLaunch> launch_;  // null: nothing to launch
+    // The prepared form, used whenever the caller's workspace holds prepared_bytes_. Null: there is none.
+    std::uint64_t prepared_bytes_{0};
+    std::shared_ptr<FtcudaGroupedGemmLaunch> prepared_;
 };
 
 }  // namespace ftrain

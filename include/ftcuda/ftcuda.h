@@ -175,12 +175,17 @@ FTCUDA_API int ftcuda_gemm_launch_scatter(const FtcudaGemmLaunch* launch, void* 
  *                               must share one operand layout class. The per-group table (TMA
  *                               descriptors, output views) is copied into the workspace by every
  *                               launch: ftcuda_grouped_gemm_workspace_bytes says how large it is.
+ *   FTCUDA_GROUPED_GEMM_FP16X3  the groups of the former that are large enough go through FTCUDA_GEMM_FP16X3, one
+ *                               after the other, the others through one FTCUDA_GROUPED_GEMM_TF32X3 launch.
+ *                               Refused when no group is large enough. The large groups take turns
+ *                               in one part of the workspace.
  * configure returns a heap object through *launch; destroy frees it (NULL is allowed).
  */
 enum {
     FTCUDA_GROUPED_GEMM_EXACT        = 0,
     FTCUDA_GROUPED_GEMM_TF32X3       = 1,
-    FTCUDA_GROUPED_GEMM_KERNEL_COUNT = 2,
+    FTCUDA_GROUPED_GEMM_FP16X3       = 2,
+    FTCUDA_GROUPED_GEMM_KERNEL_COUNT = 3,
 };
 typedef struct FtcudaGroupedGemmLaunch FtcudaGroupedGemmLaunch;
 FTCUDA_API int ftcuda_grouped_gemm_supports(int kernel, const FtcudaGemmDesc* groups, uint32_t num_groups, char* message,

@@ -126,3 +126,30 @@ def test_a_plan_offers_both_forms(capi, gpu, oracle):
     plan.execute(0, less.data_ptr(), plan.workspace_bytes(1), gpu.current_stream())
     torch.cuda.synchronize()
     check(oracle, d, a, b, None, 1.0, 0.0, "index 0 with the minimum")
+
+
+def test_grouped_plan_mixes_both_forms(capi, gpu, oracle):
+    """Large groups through the prepared form, one of them with operands it has to leave to the TF32 kernel, small ones
+    and an empty one through the one launch: index 0, the same without the workspace, and index 0 with less."""
+    torch.manual_seed(4)
+    rows, k, n = [1500, 0, 130, 1024, 40], 2048, 2048
+    groups = len(rows)
+    a, b = torch.randn(sum(rows), k, device="cuda"), torch.randn(groups * k, n, device="cuda")
+    c, d = torch.randn(sum(rows), n, device="cuda"), torch.empty(sum(rows), n, device="cuda")
+    a[7, 5] = 2.0 ** 110
+    plan = capi.GroupedGemmBinding().make_plan(
+        {"address": a.data_ptr(), "rows": rows, "cols": [k] * groups}, {"address": b.data_ptr(), "rows": [k] * groups, "cols": [n] * groups},
+        {"address": c.data_ptr(), "rows": rows, "cols": [n] * groups}, {"address": d.data_ptr(), "rows": rows, "cols": [n] * groups}, 1.5, 0.5)
+    names = plan.primitive_names()
+    assert names[0] == names[1] == "GroupedFp32Gemm3xTf32" and plan.workspace_bytes(0) > plan.workspace_bytes(1) > 0
+    workspace = torch.empty(plan.workspace_bytes(0), dtype=torch.uint8, device="cuda")
+    for index, size in ((0, plan.workspace_bytes(0)), (1, plan.workspace_bytes(1)), (0, plan.workspace_bytes(1))):
+        d.fill_(float("nan"))
+        plan.execute(index, workspace.data_ptr(), size, gpu.current_stream())
+        torch.cuda.synchronize()
+        first = 0
+        for g, m in enumerate(rows):
+            part = slice(first, first + m)
+            first += m
+            if m != 0:
+                check(oracle, d[part], a[part], b[g * k:(g + 1) * k], c[part], 1.5, 0.5, f"group {g}, index {index}, {size} bytes")
