@@ -16,7 +16,8 @@ barrier and a device synchronise, max over ranks. A, B and D together are far
 larger than the 126 MB L2, so every step streams its operands from HBM again.
 
 Roofline: the K timed steps last a fraction of a second, so `roofline.frac` is taken against the BURST
-tensor peak (measured BF16 dense / 6: TF32 = BF16/2, three products per FP32 product); `sustained` is a
+tensor peak (measured BF16 dense / 3 for the prepared form of the tensor-core Primitives: three FP16 products per FP32
+product at the BF16 rate; / 6 for the TF32 form: TF32 = BF16/2); `sustained` is a
 second leg -- the same step repeated for two seconds under the power cap, with the SM clocks sampled --
 held against the sustained peak. `tflops_per_gpu_per_ghz` divides by the sampled SM clock so that runs
 at different clocks (N = 1 against N = 8) compare.
@@ -411,6 +412,14 @@ def torch_gemm_overhead(ft_torch, torch, device) -> dict:
 
 # --------------------------------------------------------------------------- ride-along records
 
+def tensor_divisor(names, index) -> int:
+    """How many times the measured BF16 rate exceeds the FP32-product rate of a Plan's tensor-core Primitive: three FP16
+    products in the prepared form (the Plan lists the same Primitive without its workspace right behind it), three TF32
+    products at half the rate otherwise."""
+    prepared = "3xTf32" in names[index] and index + 1 < len(names) and names[index + 1] == names[index]
+    return 3 if prepared else 6
+
+
 class PlanRunner:
     """One Plan with the workspace of one of its primitives: `run()` enqueues it on torch's current stream."""
 
@@ -499,8 +508,11 @@ def config_records(torch, capi, device, peaks, ffma_tflops) -> dict:
     flops = 2.0 * 4096 ** 3
     for label, primitive, bound, peak, source in (
             ("config2_4096_cubed_addend_exact_fp32", "Fp32Gemm", "fp32", ffma_tflops, "FFMA probe measured in this run"),
-            ("config2_4096_cubed_addend_3xtf32", "Fp32Gemm3xTf32", "tensor", burst_tensor, f"{peaks['source']} bf16_tflops / 6")):
+            ("config2_4096_cubed_addend_3xtf32", "Fp32Gemm3xTf32", "tensor", None, None)):
         runner = PlanRunner(torch, a, b, c, d, 1.5, 0.5, primitive)
+        if peak is None and bound == "tensor":
+            peak   = peaks["bf16_tflops"] / tensor_divisor(runner.names, runner.index)
+            source = f"{peaks['source']} bf16_tflops / {tensor_divisor(runner.names, runner.index)}"
         stats = measure_calls(torch, runner.run)
         tflops = flops / (stats["median_us"] * 1e-6) / 1e12
         records[label] = {"primitive": runner.name, **stats, "tflops": round(tflops, 2), "bound": bound,
@@ -540,9 +552,10 @@ def config_records(torch, capi, device, peaks, ffma_tflops) -> dict:
             runner = PlanRunner(torch, a, copies[0], None, d)
             stats = measure_calls(torch, runner.run)
             tflops = 2.0 * m * 4096 * 4096 / (stats["median_us"] * 1e-6) / 1e12
+            divisor = tensor_divisor(runner.names, runner.index)
             records[f"config3_{m}x4096x4096_{label}"] = {
                 "primitive": runner.name, "workspace_bytes": runner.size, **stats, "bound": "tensor", "tflops": round(tflops, 2),
-                "frac": round(tflops / burst_tensor, 4), "peak_source": f"{peaks['source']} bf16_tflops / 6"}
+                "frac": round(tflops / (peaks["bf16_tflops"] / divisor), 4), "peak_source": f"{peaks['source']} bf16_tflops / {divisor}"}
     del copies
     # --- grouped GEMM (GroupedABCDGemm): eight "experts" with ragged token counts, one empty, x @ W_g per group
     from flash_train.capi import GroupedGemmBinding
@@ -570,8 +583,9 @@ def config_records(torch, capi, device, peaks, ffma_tflops) -> dict:
         call = lambda: grouped_plan.execute(index, workspace.data_ptr() if size else 0, size, stream)  # noqa: E731
         stats = measure_calls(torch, call)
         tflops = grouped_flops / (stats["median_us"] * 1e-6) / 1e12
-        peak, bound = (burst_tensor, "tensor") if "3xTf32" in name else (ffma_tflops, "fp32")
-        grouped[name] = {**stats, "tflops": round(tflops, 2), "bound": bound, "frac": round(tflops / peak, 4) if peak else None,
+        names = grouped_plan.primitive_names()
+        peak, bound = (peaks["bf16_tflops"] / tensor_divisor(names, index), "tensor") if "3xTf32" in name else (ffma_tflops, "fp32")
+        grouped[name + ("_without_its_workspace" if index and names[index - 1] == name else "")] = {**stats, "tflops": round(tflops, 2), "bound": bound, "frac": round(tflops / peak, 4) if peak else None,
                          "workspace_bytes": size}
     # The same products as separate Plans of the plain Gemm, one launch each, for comparison.
     singles = [PlanRunner(torch, tokens[s:s + count], weights[g], None, result[s:s + count])
@@ -712,7 +726,7 @@ def k_split_records(torch, capi, world, rank, device, steps: int, peaks) -> dict
                                 "reduce_scatter_ms": collective_ms, "collective_share": collective_ms / step_ms,
                                 "timed": "whole step, local GEMM alone and reduce_scatter_tensor alone, each in its own event-timed loop "
                                          "(maximum over ranks); the loops run one after another, so clocks under the power cap differ a little",
-                                "frac_of_burst_tensor_peak_per_gpu": flops / (step_ms * 1e-3) / 1e12 / world / (peaks["bf16_tflops"] / 6.0),
+                                "frac_of_burst_tensor_peak_per_gpu": flops / (step_ms * 1e-3) / 1e12 / world / (peaks["bf16_tflops"] / 3.0),
                                 **parity(out)}
     try:
         os.environ.setdefault("TORCH_SYMM_MEM_DISABLE_MULTICAST", "1")  # plain peer mappings, no NVLink multicast object
@@ -916,7 +930,9 @@ def run_k_split(options, torch, capi, world, rank, local_rank, device) -> int:
         ms_per_step = elapsed_ms / options.steps
         value = 2.0 * m * n * k / (ms_per_step * 1e-3) / 1e12
         peaks = measured_peaks()
-        tensor_peak = peaks["bf16_tflops"] / 6.0
+        # The local Plan runs the prepared form (three FP16 products), the adding launch the TF32 one.
+        divisor = 6 if distributed and options.workload == KSPLIT_FUSED_WORKLOAD else 3
+        tensor_peak = peaks["bf16_tflops"] / divisor
         line = {
             "metric": "fp32_gemm_tflops", "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": options.steps,
             "warmup": options.warmup, "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "strong",
@@ -926,7 +942,7 @@ def run_k_split(options, torch, capi, world, rank, local_rank, device) -> int:
                        "l2": "A and B shards (2 x 2 GiB in total) exceed the 126 MB L2"},
             "roofline": {"bound": "tensor", "achieved": value / world, "peak": tensor_peak, "unit": "TFLOP/s",
                          "frac": value / world / tensor_peak, "traffic": None,
-                         "peak_source": f"{peaks['source']} bf16_tflops / 6 (burst: the timed region is well under a second)"},
+                         "peak_source": f"{peaks['source']} bf16_tflops / {divisor} (burst: the timed region is well under a second)"},
             "tflops_per_gpu_per_ghz": per_ghz(value / world, clocks),
             "clocks": clocks, "gpu_launches": launches,
         }
@@ -1126,18 +1142,21 @@ def main() -> int:
                 ffma_tflops = max(ffma_tflops or 0.0, capi.measure_ffma_tflops(local_rank))
         ffma_clocks = ffma_sampler.summary()
     if tensor_kernel:
-        burst_peak = peaks["bf16_tflops"] / 6.0
-        traffic = MEASURED_DRAM_TRAFFIC.get((options.workload, primitive, world))
+        divisor = tensor_divisor(plan_names, index)
+        burst_peak = peaks["bf16_tflops"] / divisor
+        # The captures are of the TF32 kernel.
+        traffic = MEASURED_DRAM_TRAFFIC.get((options.workload, primitive, world)) if divisor == 6 else None
         roofline = {"bound": "tensor", "achieved": per_gpu, "peak": burst_peak, "unit": "TFLOP/s",
                     "frac": per_gpu / burst_peak, "traffic": traffic, "traffic_source": TRAFFIC_SOURCE if traffic else None,
                     "algorithmic_bytes": 4 * (m * k + k * n + m * n * (2 if with_c else 1)),
-                    "peak_source": f"{peaks['source']} bf16_tflops / 6 (burst; TF32 = BF16/2; 3 MMAs per product): "
+                    "peak_source": f"{peaks['source']} bf16_tflops / {divisor} (burst; "
+                                   f"{'3 FP16 products' if divisor == 3 else 'TF32 = BF16/2; 3 products'} per FP32 product): "
                                    f"{options.steps} steps of {ms_per_step:.2f} ms are a burst",
-                    "kernel": "tensorGemm3xTf32", "ms_per_launch": ms_per_step}
+                    "kernel": "splitOperands + tensorGemm3xFp16" if divisor == 3 else "tensorGemm3xTf32", "ms_per_launch": ms_per_step}
         if sustained is not None:
-            sustained_peak = peaks["bf16_tflops_sustained"] / 6.0
+            sustained_peak = peaks["bf16_tflops_sustained"] / divisor
             sustained.update({"peak": sustained_peak, "frac": sustained["value"] / world / sustained_peak,
-                              "peak_source": f"{peaks['source']} bf16_tflops_sustained / 6",
+                              "peak_source": f"{peaks['source']} bf16_tflops_sustained / {divisor}",
                               "tflops_per_gpu_per_ghz": per_ghz(sustained["value"] / world, sustained["clocks"])})
     else:
         roofline = {"bound": "fp32", "achieved": per_gpu, "peak": ffma_tflops, "unit": "TFLOP/s",
