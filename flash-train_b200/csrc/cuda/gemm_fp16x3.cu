@@ -82,7 +82,7 @@ struct Barriers {
     std::uint64_t flush_x, flush_h;
     std::uint32_t tmem_base;
     int abort_flag;
-    std::uint32_t few[2][3], flags;  // the worst of the verdicts
+    std::uint32_t few[2][2][3], flags[2];  // the worst verdicts: whole slabs' and a shorter last slab's, A's and B's
 };
 static_assert(sizeof(Barriers) <= 256, "barrier block");
 
@@ -102,6 +102,9 @@ struct Fp16Params {
     std::uint64_t inverse_pitch_a, inverse_pitch_b;
     const std::uint32_t* verdicts;  // of the split's CTAs: first A's, then B's
     std::uint32_t verdicts_a, verdicts_b;
+    std::uint32_t slabs;
+    std::uint32_t slabs_fastest;    // bit 0: A's verdicts run through the slabs first (else slab by slab), bit 1: B's
+    std::uint32_t short_slab;       // the last slab is shorter than the others
     std::uint32_t* use_fallback;    // the decision, for the kernels behind this one
     std::uint32_t vector;  // consecutive columns of the output and C that one aligned access takes: 8, 4, or 0 (any strides)
     int* status;
@@ -264,8 +267,8 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         mbarrierInit(&bars->flush_x, 1);
         mbarrierInit(&bars->flush_h, 1);
         bars->abort_flag = 0;
-        for (int i = 0; i < 6; ++i) { bars->few[i / 3][i % 3] = 0; }
-        bars->flags = 0;
+        for (int i = 0; i < 12; ++i) { bars->few[i / 6][i / 3 % 2][i % 3] = 0; }
+        bars->flags[0] = bars->flags[1] = 0;
         fenceBarrierInit();
         prefetchTensorMap(&map_a);
         prefetchTensorMap(&map_b);
@@ -283,32 +286,48 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     gridDependencyLaunchDependents();
     // Every CTA comes to the same decision. Left to the fallback, there are no items.
     {
-        std::uint32_t flags = 0;
+        // A gray element only concerns its own slab. A shorter last slab is kept apart from the others: of a handful of K
+        // values a column can well have none of full size, and a gray element elsewhere is no reason to mind.
         for (int which = 0; which < 2; ++which) {
             const std::uint32_t* const verdicts = p.verdicts + (which != 0 ? p.verdicts_a : 0);
             const std::uint32_t count           = which != 0 ? p.verdicts_b : p.verdicts_a;
-            std::uint32_t few[3]                = {0, 0, 0};
+            const bool slabs_fastest            = (p.slabs_fastest >> which & 1U) != 0;
+            const std::uint32_t last_slab_at    = count - count / p.slabs;
+            std::uint32_t few[2][3] = {{0, 0, 0}, {0, 0, 0}}, flags[2] = {0, 0};
 #pragma unroll 4
             for (std::uint32_t i = threadIdx.x; i < count; i += kThreads) {
                 const std::uint32_t verdict = __ldcg(verdicts + i);
-                flags |= verdict;
+                const bool in_last = p.short_slab != 0 && (slabs_fastest ? i % p.slabs == p.slabs - 1 : i >= last_slab_at);
+                flags[0] |= in_last ? 0U : verdict;
+                flags[1] |= in_last ? verdict : 0U;
 #pragma unroll
-                for (int t = 0; t < 3; ++t) { few[t] = max(few[t], verdict >> (10 * t) & fp16x3::kVerdictFew); }
+                for (int t = 0; t < 3; ++t) {
+                    const std::uint32_t small = verdict >> (10 * t) & fp16x3::kVerdictFew;
+                    few[0][t] = max(few[0][t], in_last ? 0U : small);
+                    few[1][t] = max(few[1][t], in_last ? small : 0U);
+                }
             }
 #pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                few[t] = __reduce_max_sync(0xFFFFFFFFU, few[t]);
-                if (lane == 0) { atomicMax(&bars->few[which][t], few[t]); }
+            for (int kind = 0; kind < 2; ++kind) {
+                flags[kind] = __reduce_or_sync(0xFFFFFFFFU, flags[kind]);
+                if (lane == 0) { atomicOr(&bars->flags[kind], flags[kind]); }
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    few[kind][t] = __reduce_max_sync(0xFFFFFFFFU, few[kind][t]);
+                    if (lane == 0) { atomicMax(&bars->few[kind][which][t], few[kind][t]); }
+                }
             }
         }
-        flags = __reduce_or_sync(0xFFFFFFFFU, flags);
-        if (lane == 0) { atomicOr(&bars->flags, flags); }
         __syncthreads();
-        // F_a + F_b - 1 >= 1/64, in 1023rds of a slab and with one to spare for the rounding of each, for any pair
-        // of thresholds whose exponents add up to 18.
-        const auto enough = [&](int a, int b) { return bars->few[0][a] + bars->few[1][b] + 16 + 2 <= 1023; };
-        const bool fallback = (bars->flags & fp16x3::kVerdictOutOfRange) != 0 ||
-                              ((bars->flags & fp16x3::kVerdictGray) != 0 && !enough(0, 2) && !enough(1, 1) && !enough(2, 0));
+        bool fallback = false;
+#pragma unroll
+        for (int kind = 0; kind < 2; ++kind) {
+            // F_a + F_b - 1 >= 1/64, in 1023rds of a slab and with one to spare for the rounding of each, for any pair
+            // of thresholds whose exponents add up to 18.
+            const auto enough = [&](int a, int b) { return bars->few[kind][0][a] + bars->few[kind][1][b] + 16 + 2 <= 1023; };
+            fallback = fallback || (bars->flags[kind] & fp16x3::kVerdictOutOfRange) != 0 ||
+                       ((bars->flags[kind] & fp16x3::kVerdictGray) != 0 && !enough(0, 2) && !enough(1, 1) && !enough(2, 0));
+        }
         if (blockIdx.x == 0 && threadIdx.x == 0) { *p.use_fallback = fallback ? 1U : 0U; }
         if (fallback) { num_items = 0; }
     }
@@ -662,6 +681,9 @@ cudaError_t launchPrepared(const LaunchState& state, void* workspace, cudaStream
     p.verdicts         = verdicts;
     p.verdicts_a       = split.operand[0].blocks;
     p.verdicts_b       = split.operand[1].blocks;
+    p.slabs            = split.slabs;
+    p.slabs_fastest    = split.operand[0].along_k | split.operand[1].along_k << 1;
+    p.short_slab       = split.k % fp16x3::kSlabK != 0 ? 1U : 0U;
     p.use_fallback     = decision;
     p.status           = state.device_status;
     const auto aligned = [&](std::uint32_t width, const float* at, std::int64_t row_stride, std::int64_t col_stride) {

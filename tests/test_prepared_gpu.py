@@ -109,6 +109,27 @@ def test_operands_left_to_the_tf32_kernel(capi, gpu, kind):
         assert torch.equal(one.view(torch.int32), other.view(torch.int32)), kind
 
 
+@pytest.mark.parametrize("k", [768, 769, 775, 1536 + 64])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_a_gray_element_concerns_its_own_slab_only(capi, gpu, oracle, k, transposed):
+    """A tiny element among full ones does not cost the prepared form, however short the last slab is; it does where its
+    slab holds too few full ones beside it."""
+    torch.manual_seed(k)
+    m, n = 520, 900
+    a, b = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda")
+    a[5, 3] = 2.0 ** -40
+    a_view, b_view = (a.t().contiguous().t(), b.t().contiguous().t()) if transposed else (a, b)
+    d = run(capi, gpu, capi.KERNEL_FP16X3, a_view, b_view, None, 1.0, 0.0)
+    check(oracle, d, a, b, None, 1.0, 0.0, "tiny element")
+    assert not torch.equal(d, run(capi, gpu, capi.KERNEL_TF32X3, a_view, b_view, None, 1.0, 0.0)), "went to the TF32 kernel"
+    b[:700, 7] *= 2.0 ** -20  # ... and now a column has hardly any full element where the row's tiny one is
+    b_view = b.t().contiguous().t() if transposed else b
+    a[:, :700] *= torch.where(torch.arange(700, device="cuda") % 2 == 0, 1.0, 2.0 ** -20)
+    a_view = a.t().contiguous().t() if transposed else a
+    assert torch.equal(run(capi, gpu, capi.KERNEL_FP16X3, a_view, b_view, None, 1.0, 0.0),
+                       run(capi, gpu, capi.KERNEL_TF32X3, a_view, b_view, None, 1.0, 0.0)), "kept the FP16 kernel"
+
+
 def test_a_plan_offers_both_forms(capi, gpu, oracle):
     """Index 0 asks for the prepared form's workspace, the same Primitive without it follows, and index 0 still
     runs with less."""
