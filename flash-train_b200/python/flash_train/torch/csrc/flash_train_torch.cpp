@@ -150,7 +150,8 @@ bool planReuseDisabled() {
 
 // Runs the Plan's first primitive whose workspace torch's allocator can give: the best form of a tensor-core
 // family takes as much memory as A and B, and the primitives behind it do with less.
-FTrainStatus executePlan(FTrainPlan plan, std::uint64_t first_bytes, const at::TensorOptions& options, FTrainStream stream) {
+FTrainStatus executePlan(FTrainPlan plan, std::uint64_t first_bytes, const at::Tensor& like, FTrainStream stream) {
+    if (first_bytes == 0) { return ftrainPlanExecutePrimitive(plan, 0, nullptr, 0, stream); }
     std::uint64_t bytes = first_bytes;
     for (std::uint64_t index = 0;; ++index) {
         if (index != 0) {
@@ -160,7 +161,7 @@ FTrainStatus executePlan(FTrainPlan plan, std::uint64_t first_bytes, const at::T
         at::Tensor workspace;
         if (bytes != 0) {
             try {
-                workspace = torch::empty({static_cast<std::int64_t>(bytes)}, options.dtype(at::kByte));
+                workspace = torch::empty({static_cast<std::int64_t>(bytes)}, like.options().dtype(at::kByte));
             } catch (const c10::OutOfMemoryError&) {
                 std::uint64_t count = 0;
                 if (ftrainPlanGetNumPrimitives(plan, &count) != FTRAIN_STATUS_SUCCESS || index + 1 >= count) { throw; }
@@ -212,7 +213,7 @@ at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const std::optional<at
     key.device = a.device().index();
     if (reuse) {
         if (RecentPlans::Entry* known = recent.find(key)) {
-            const FTrainStatus again = executePlan(known->plan, known->workspace_bytes, a.options(), stream);
+            const FTrainStatus again = executePlan(known->plan, known->workspace_bytes, a, stream);
             TORCH_CHECK(again == FTRAIN_STATUS_SUCCESS, "flash_train gemm failed with status ", static_cast<unsigned>(again), ": ",
                         ftrainGetLastMessage());
             return d;
@@ -241,7 +242,7 @@ at::Tensor gemm(const at::Tensor& a, const at::Tensor& b, const std::optional<at
     if (status == FTRAIN_STATUS_SUCCESS) { status = ftrainPlanCreate(&plan, args); }
     std::uint64_t workspace_bytes = 0;
     if (status == FTRAIN_STATUS_SUCCESS) { status = ftrainPlanGetPrimitiveRequiredWorkspaceBytes(plan, 0, &workspace_bytes); }
-    if (status == FTRAIN_STATUS_SUCCESS) { status = executePlan(plan, workspace_bytes, a.options(), stream); }
+    if (status == FTRAIN_STATUS_SUCCESS) { status = executePlan(plan, workspace_bytes, a, stream); }
     const std::string failure = status == FTRAIN_STATUS_SUCCESS ? std::string() : std::string(ftrainGetLastMessage());
     if (status == FTRAIN_STATUS_SUCCESS && reuse) {
         recent.insert(key, plan, workspace_bytes);  // kept for the next call with these tensors
