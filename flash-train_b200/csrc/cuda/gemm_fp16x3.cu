@@ -20,7 +20,7 @@
 //
 // Tensor memory holds two accumulators, 512 columns in all: X, the two cross products, issued by warp 1, and H, a_hi b_hi,
 // issued by warp 2. Both are read at the end of every slab of K (768, the split's unit of scaling), multiplied by
-// the slab's powers of two -- exactly -- and added up in registers, to nearest. The tensor core's own FP32
+// the slab's powers of two (addScaled) and added up in registers, to nearest. The tensor core's own FP32
 // additions truncate, so for a small K H is read more often than that (chunkBlocks); X is 2^11 times smaller
 // in effect. With an issuer each, one accumulator is read while products go to the other, and what a single thread does
 // between two K blocks -- barriers, descriptors -- no longer leaves the tensor pipe idle (one issuer for both:
@@ -219,8 +219,12 @@ __device__ __forceinline__ void writePiece(const Fp16Params& p, const Item& w, s
     }
 }
 
-// acc += row_scale * scale of the 16 columns * accumulator, for up to four pieces of 32 columns at `tmem`. The products
-// of powers of two are exact.
+// acc += row_scale * scale of the 16 columns * accumulator, for up to four pieces of 32 columns at `tmem`. The scales are powers
+// of two. As long as their product is one that FP32 has (not under 2^-149), it scales exactly and the addition is the only
+// rounding. Operands may be as small as 2^-100 each, so it need not be: then (kApart) the row's scale, which alone is at least
+// 2^-125, is applied first. What that rounds off is under 2^-150 / 2^-125 of one in units of the accumulator, whose
+// products reach up to 2^28. Twice the arithmetic, so only where it is needed.
+template<bool kApart>
 __device__ __forceinline__ void addScaled(std::uint32_t tmem, std::uint32_t pieces, float row_scale, const float (&scales)[8],
                                           float2 (&acc)[64]) {
 #pragma unroll
@@ -230,11 +234,13 @@ __device__ __forceinline__ void addScaled(std::uint32_t tmem, std::uint32_t piec
             tmemLoad32(tmem + q * 32, v);
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
-                const float scale = row_scale * scales[2 * q + g];
+                const float scale = kApart ? scales[2 * q + g] : row_scale * scales[2 * q + g];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    float2& sum = acc[q * 16 + g * 8 + j];
-                    sum = multiplyAdd2(make_float2(scale, scale), make_float2(v[g * 16 + 2 * j], v[g * 16 + 2 * j + 1]), sum);
+                    float2& sum  = acc[q * 16 + g * 8 + j];
+                    float2 value = make_float2(v[g * 16 + 2 * j], v[g * 16 + 2 * j + 1]);
+                    if (kApart) { value = multiply2(make_float2(row_scale, row_scale), value); }
+                    sum = multiplyAdd2(make_float2(scale, scale), value, sum);
                 }
             }
         }
@@ -353,13 +359,16 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             for (int j = 0; j < 64; ++j) { acc[j] = make_float2(0.0F, 0.0F); }
             for (std::uint32_t block = 0, in_slab; block < w.blocks && ok; block += in_slab, ++slabs) {
                 in_slab = blocksInSlab(w, block);
-                // The slab's scales: of this thread's row, and of this warp's groups of 16 columns.
+                // The slab's scales: of this thread's row, and of this warp's groups of 16 columns (1 beyond the last).
                 const std::uint32_t slab = (w.first_block + block) / kSlabBlocks;
-                const float row_scale    = p.inverse_a[slab * p.inverse_pitch_a + row0 + lane];
+                const float row_scale    = row0 + lane < p.m ? p.inverse_a[slab * p.inverse_pitch_a + row0 + lane] : 1.0F;
                 const float* const groups = p.inverse_b + slab * p.inverse_pitch_b + mine_at / fp16x3::kColumnGroup;
                 float scales[8];
 #pragma unroll
-                for (int g = 0; g < 8; ++g) { scales[g] = groups[g]; }
+                for (std::uint32_t g = 0; g < 8; ++g) { scales[g] = mine_at + g * fp16x3::kColumnGroup < p.n ? groups[g] : 1.0F; }
+                const float smallest = fminf(fminf(fminf(scales[0], scales[1]), fminf(scales[2], scales[3])),
+                                             fminf(fminf(scales[4], scales[5]), fminf(scales[6], scales[7])));
+                const bool apart     = __any_sync(0xFFFFFFFFU, row_scale * 0x1p-11F * smallest == 0.0F);
                 const std::uint32_t num_chunks = (in_slab + p.chunk_blocks - 1) / p.chunk_blocks;
                 for (std::uint32_t chunk = 0; chunk < num_chunks && ok; ++chunk, ++chunks) {
                     // X once per slab, ahead of the last reading of H.
@@ -367,7 +376,11 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         ok = mbarrierWait(&bars->x_full, slabs & 1, abort_flag);
                         if (!ok) { break; }
                         tcgen05FenceAfterSync();
-                        addScaled(tmem_row + first * 32, mine, row_scale * 0x1p-11F, scales, acc);
+                        if (apart) {
+                            addScaled<true>(tmem_row + first * 32, mine, row_scale * 0x1p-11F, scales, acc);
+                        } else {
+                            addScaled<false>(tmem_row + first * 32, mine, row_scale * 0x1p-11F, scales, acc);
+                        }
                         tcgen05FenceBeforeSync();
                         __syncwarp();
                         if (lane == 0) { mbarrierArriveCluster(x_empty); }
@@ -375,7 +388,11 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     ok = mbarrierWait(&bars->h_full, chunks & 1, abort_flag);
                     if (!ok) { break; }
                     tcgen05FenceAfterSync();
-                    addScaled(tmem_row + kHColumn + first * 32, mine, row_scale, scales, acc);
+                    if (apart) {
+                        addScaled<true>(tmem_row + kHColumn + first * 32, mine, row_scale, scales, acc);
+                    } else {
+                        addScaled<false>(tmem_row + kHColumn + first * 32, mine, row_scale, scales, acc);
+                    }
                     tcgen05FenceBeforeSync();
                     __syncwarp();
                     if (lane == 0) { mbarrierArriveCluster(h_empty); }
@@ -599,8 +616,7 @@ int configurePrepared(LaunchState& state, const FtcudaGemmDesc& desc, char* mess
     prepared.verdicts_at        = at;
     at += roundUp((static_cast<std::uint64_t>(operands[0].blocks) + operands[1].blocks) * 4, 256);
     for (int i = 0; i < 2; ++i) {
-        // A tile reads its scales beyond the last row, too (and does not use them).
-        prepared.inverse_pitch[i] = roundUp((rows[i] + 2 * kMaxTileN) / (i == 0 ? 1 : fp16x3::kColumnGroup), 4);
+        prepared.inverse_pitch[i] = roundUp(ceilDiv(rows[i], i == 0 ? 1 : fp16x3::kColumnGroup), 4);
         prepared.inverse_at[i]    = at;
         at += roundUp(slabs * prepared.inverse_pitch[i] * 4, 256);
     }

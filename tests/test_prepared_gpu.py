@@ -77,6 +77,21 @@ def test_scales_of_rows_and_columns(capi, gpu, oracle):
     assert ((d.double() - exact).abs() <= bound).all() and (d[7] == 0).all() and (d[:, 11] == 0).all()
 
 
+@pytest.mark.parametrize("exponent_a,exponent_b", [(-55, -55), (-57, -57), (-63, -63), (-90, -30), (-30, -90), (-98, 55)])
+@pytest.mark.parametrize("m,k,n", [(300, 1600, 270), (129, 5000, 130)])  # without and with K slices
+def test_products_of_small_magnitude(capi, gpu, m, k, n, exponent_a, exponent_b):
+    """The inverse scales of a row and of a column may each be a normal number and their product not: the results are
+    normal numbers all the same, also when a large alpha brings them to an ordinary size."""
+    torch.manual_seed(k)
+    a, b = torch.randn(m, k, device="cuda") * 2.0 ** exponent_a, torch.randn(k, n, device="cuda") * 2.0 ** exponent_b
+    for alpha in (1.0, 2.0 ** 60):
+        exact = alpha * (a.double() @ b.double())
+        prepared, plain = (run(capi, gpu, kernel, a, b, None, alpha, 0.0) for kernel in (capi.KERNEL_FP16X3, capi.KERNEL_TF32X3))
+        ours, other = (((d.double() - exact).norm() / exact.norm()).item() for d in (prepared, plain))
+        assert ours <= 2.0 * max(other, ERROR_FLOOR), f"alpha {alpha}: {ours:.3e} against {other:.3e} of the TF32 form"
+        assert not torch.equal(prepared, plain), "went to the TF32 kernel"
+
+
 @pytest.mark.parametrize("kind", ["depth", "pair", "sparse", "large", "tiny", "inf", "nan"])
 def test_operands_left_to_the_tf32_kernel(capi, gpu, kind):
     """Magnitudes that spread too far for scaled FP16 pairs (or are not finite): the result is bit for bit that of
