@@ -56,12 +56,39 @@ def k_range(k: int, world: int, rank: int, granule: int = K_GRANULE) -> Tuple[in
 class _LibraryGemm:
     """d = alpha * a @ b + beta * c through one reusable Plan per (addresses, scalars)."""
 
+    # Calls that do without a workspace as large as one the allocator could not give, before it is asked again (each
+    # refusal makes it synchronise the device and give back all that it caches).
+    ASK_AGAIN_AFTER = 64
+
     def __init__(self):
         from . import capi
 
         self._capi = capi
         self._binding = capi.GemmBinding()
         self._plans = {}
+        self._refused_bytes, self._refused_calls = 0, 0
+
+    def _workspace(self, sizes, device):
+        """(index, workspace) of the first primitive whose workspace torch's allocator can give: the best form of a
+        tensor-core family takes as much memory as A and B, and the primitives behind it do with less.
+
+        From the caching allocator on every call: the block belongs to the current stream, and the Plans kept here do
+        not each hold one."""
+        import torch
+
+        last = len(sizes) - 1
+        if self._refused_calls and sizes[0] >= self._refused_bytes:
+            self._refused_calls -= 1
+        for index, size in enumerate(sizes):
+            if index < last and self._refused_calls and size >= self._refused_bytes:
+                continue
+            try:
+                return index, torch.empty(max(size, 1), dtype=torch.uint8, device=device)
+            except torch.OutOfMemoryError:
+                if index == last:
+                    raise
+                self._refused_bytes, self._refused_calls = size, self.ASK_AGAIN_AFTER
+        raise AssertionError("a Plan holds at least one primitive")
 
     def __call__(self, a, b, c, d, alpha: float, beta: float) -> None:
         import torch
@@ -76,14 +103,12 @@ class _LibraryGemm:
                 capi.tensor_operand(a), capi.tensor_operand(b),
                 capi.tensor_operand(c) if c is not None else capi.null_operand(rows, cols),
                 capi.tensor_operand(d), alpha, beta)
-            size = plan.workspace_bytes(0)
-            entry = (plan, size)
+            entry = (plan, [plan.workspace_bytes(index) for index in range(plan.num_primitives)])
             self._plans[key] = entry
-        plan, size = entry
-        # From the caching allocator on every call: the block belongs to the current stream, and the
-        # Plans kept here do not each hold one.
-        workspace = torch.empty(max(size, 1), dtype=torch.uint8, device=a.device)
-        plan.execute(0, workspace.data_ptr() if size else 0, size, torch.cuda.current_stream(a.device).cuda_stream)
+        plan, sizes = entry
+        index, workspace = self._workspace(sizes, a.device)
+        size = sizes[index]
+        plan.execute(index, workspace.data_ptr() if size else 0, size, torch.cuda.current_stream(a.device).cuda_stream)
 
 
 LocalGemm = Callable[..., None]

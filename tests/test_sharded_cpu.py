@@ -95,3 +95,49 @@ def test_two_ranks_match_the_unsplit_product(oracle):
     assert np.array_equal(d_rows, expected)
     # K split: another summation order, and beta * C added exactly once.
     assert np.allclose(d_split, expected, rtol=1e-5, atol=1e-5)
+
+
+def test_a_workspace_the_allocator_refuses_is_done_without(capi, monkeypatch):
+    """Index 0 of a Plan may ask for as much memory as the operands: on a full GPU the next index that fits runs, and the
+    allocator is not asked for the large block on every call. What no index can do without is an error, as ever."""
+    from flash_train import sharded
+
+    limit, asked, ran = [5000], [], []
+    real_empty = torch.empty
+
+    def empty(size, **kwargs):
+        asked.append(size)
+        if size > limit[0]:
+            raise torch.OutOfMemoryError("out of memory")
+        return real_empty(size, dtype=kwargs["dtype"])
+
+    class FakePlan:
+        sizes = [100000, 6000, 4000, 0]
+        num_primitives = len(sizes)
+
+        def workspace_bytes(self, index):
+            return self.sizes[index]
+
+        def execute(self, index, workspace, size, stream):
+            ran.append((index, size, workspace != 0))
+
+    class FakeStream:
+        cuda_stream = 0
+
+    a, b, d = torch.zeros(4, 3), torch.zeros(3, 5), torch.zeros(4, 5)
+    monkeypatch.setattr(torch, "empty", empty)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: FakeStream)
+    gemm = sharded._LibraryGemm()
+    monkeypatch.setattr(gemm._binding, "make_plan", lambda *operands: FakePlan())
+    for _ in range(3):
+        gemm(a, b, None, d, 1.0, 0.0)
+    assert ran == [(2, 4000, True)] * 3 and asked == [100000, 6000, 4000, 4000, 4000]
+    asked.clear(), ran.clear()
+    limit[0] = 10 ** 6  # memory is back: found out after a while
+    for _ in range(gemm.ASK_AGAIN_AFTER):
+        gemm(a, b, None, d, 1.0, 0.0)
+    assert ran[0] == (2, 4000, True) and ran[-1] == (0, 100000, True) and asked[-1] == 100000
+    limit[0] = 0
+    FakePlan.sizes, FakePlan.num_primitives = [100000, 7000], 2
+    with pytest.raises(torch.OutOfMemoryError):
+        gemm(a, b, None, d, 2.0, 0.0)  # other scalars, another Plan
