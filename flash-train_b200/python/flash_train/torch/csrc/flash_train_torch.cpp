@@ -12,7 +12,8 @@
 //     split-K kernel that needs one, so the binding makes the same staged calls
 //     ftrainGemm makes (Args, Plan, execute primitive 0) and, in between, asks
 //     the Plan how much workspace primitive 0 wants and takes it from torch's
-//     caching allocator;
+//     caching allocator, or, where that has no block as large, does the same
+//     with the primitives behind it;
 //   * a failure carries the library's diagnostic message, not only the status;
 //   * the Plans of recent calls are kept per thread (64, least recently used out first), keyed by
 //     the four addresses, the shape, alpha, beta and the device: a training loop that calls with
@@ -28,6 +29,7 @@
 #include <cstring>
 #include <optional>
 #include <string>
+#include <vector>
 
 #include <flash_train/env.h>
 #include <flash_train/flash_train.h>
@@ -148,11 +150,28 @@ bool planReuseDisabled() {
     return disabled;
 }
 
+// A size that torch's allocator could not give this thread on a device, and for how many more calls nothing as large is asked
+// for: each refusal makes the allocator synchronise the device and give back all that it caches, which a program near
+// the end of the memory would pay on every call. Not kept with a Plan: such a program's addresses, and with them its Plans, change.
+struct RefusedWorkspace {
+    std::uint64_t bytes = 0;
+    unsigned calls      = 0;
+};
+constexpr unsigned kAskAgainAfter = 64;
+
+RefusedWorkspace& refusedWorkspace(std::size_t device) {
+    static thread_local std::vector<RefusedWorkspace> refused;
+    if (refused.size() <= device) { refused.resize(device + 1); }
+    return refused[device];
+}
+
 // Runs the Plan's first primitive whose workspace torch's allocator can give: the best form of a tensor-core
 // family takes as much memory as A and B, and the primitives behind it do with less.
 FTrainStatus executePlan(FTrainPlan plan, std::uint64_t first_bytes, const at::Tensor& like, FTrainStream stream) {
     if (first_bytes == 0) { return ftrainPlanExecutePrimitive(plan, 0, nullptr, 0, stream); }
-    std::uint64_t bytes = first_bytes;
+    RefusedWorkspace& refused = refusedWorkspace(static_cast<std::size_t>(like.device().index()));
+    if (refused.calls != 0 && first_bytes >= refused.bytes) { --refused.calls; }
+    std::uint64_t bytes = first_bytes, count = 0;
     for (std::uint64_t index = 0;; ++index) {
         if (index != 0) {
             const FTrainStatus status = ftrainPlanGetPrimitiveRequiredWorkspaceBytes(plan, index, &bytes);
@@ -160,11 +179,16 @@ FTrainStatus executePlan(FTrainPlan plan, std::uint64_t first_bytes, const at::T
         }
         at::Tensor workspace;
         if (bytes != 0) {
+            const auto more = [&] {
+                if (count == 0 && ftrainPlanGetNumPrimitives(plan, &count) != FTRAIN_STATUS_SUCCESS) { count = 1; }
+                return index + 1 < count;
+            };
+            if (refused.calls != 0 && bytes >= refused.bytes && more()) { continue; }
             try {
                 workspace = torch::empty({static_cast<std::int64_t>(bytes)}, like.options().dtype(at::kByte));
             } catch (const c10::OutOfMemoryError&) {
-                std::uint64_t count = 0;
-                if (ftrainPlanGetNumPrimitives(plan, &count) != FTRAIN_STATUS_SUCCESS || index + 1 >= count) { throw; }
+                if (!more()) { throw; }
+                refused = RefusedWorkspace{bytes, kAskAgainAfter};
                 continue;
             }
         }

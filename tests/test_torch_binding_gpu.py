@@ -63,3 +63,33 @@ def test_rejections_raise_runtime_error(binding):
         binding.gemm(a.to(torch.float64), b)
     with pytest.raises(RuntimeError):
         binding.gemm(a.t(), b)  # not contiguous: rejected by the binding, as in the reference
+
+
+def test_a_workspace_the_allocator_refuses_is_not_asked_for_on_every_call(binding):
+    """With too little memory for the prepared form's workspace the result is that of the form without it, and the allocator,
+    which gives back all that it caches at each refusal, is asked once for many calls, whatever their addresses."""
+    m = k = n = 2048
+    generator = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.randn(m, k, device="cuda", generator=generator)
+    b = torch.randn(k, n, device="cuda", generator=generator)
+    full = binding.gemm(a, b)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    out_bytes = 4 * m * n  # the prepared form's workspace takes more than two of these; two and a half are left
+    total = torch.cuda.get_device_properties(a.device).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 2.5 * out_bytes) / total)
+    try:
+        before = torch.cuda.memory_stats()["num_alloc_retries"]
+        lean = None
+        for _ in range(20):
+            lean = binding.gemm(a, b)  # the last result is still held: addresses alternate
+        torch.cuda.synchronize()
+        refusals = torch.cuda.memory_stats()["num_alloc_retries"] - before
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert 1 <= refusals <= 3  # one for each size of the Plan's workspaces
+    assert not torch.equal(full, lean), "the prepared form ran after all"
+    torch.testing.assert_close(lean, a @ b, rtol=1e-4, atol=1e-3)
+    for _ in range(80):  # memory is back: the prepared form is found again
+        last = binding.gemm(a, b)
+    assert torch.equal(last, full)
