@@ -24,12 +24,17 @@ constexpr std::uint32_t kSplitRows       = 32;
 
 constexpr std::uint32_t kColumnGroup = 16;  // columns of B that share a scale
 
-// What one CTA of the split found: how many elements of a row are below 2^-5, 2^-9 and 2^-13 of the largest
-// its scale allows for, in 1023rds of the slab (the worst row; ten bits each), an element far below that, a row
-// whose magnitudes the scaling does not cover.
-constexpr std::uint32_t kVerdictFew        = 0x3FF;
-constexpr std::uint32_t kVerdictGray       = 1U << 30;
-constexpr std::uint32_t kVerdictOutOfRange = 1U << 31;
+// What one CTA of the split found, a word for each slab and group of rows: how many nonzero rows' elements are below 2^-5, 2^-9
+// and 2^-13 of the largest the row's scale allows for (the worst row; ten bits each), and what else there is to mind.
+constexpr std::uint32_t kVerdictSmall = 0x3FF;
+constexpr int kVerdictState           = 30;
+enum VerdictState : std::uint32_t {
+    kAllCovered  = 0,
+    kFewGray     = 1,  // elements far below that, up to kFewGrayElements in a row
+    kManyGray    = 2,
+    kOutOfRange  = 3,  // a row whose magnitudes the scaling does not cover
+};
+constexpr std::uint32_t kFewGrayElements = 64;
 
 struct SplitOperand {
     const float* source;
@@ -43,7 +48,7 @@ struct SplitOperand {
     unsigned char* split;
     float* inverse;           // [slab][pitch]: 1 / (scale of the row or group in the slab), a power of two
     std::uint64_t pitch;
-    std::uint32_t* verdicts;  // [blocks]
+    std::uint32_t* verdicts;  // [slab][blocks / slabs]
 };
 
 struct SplitParams {

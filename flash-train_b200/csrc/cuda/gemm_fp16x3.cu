@@ -53,6 +53,7 @@ namespace {
 using fp16x3::kBlockBytes;
 using fp16x3::kBlockK;
 using fp16x3::kSlabBlocks;
+using fp16x3::kSlabK;
 
 constexpr int kTileM      = 256;  // of a CTA pair
 constexpr int kMaxTileN   = 256;
@@ -82,7 +83,7 @@ struct Barriers {
     std::uint64_t flush_x, flush_h;
     std::uint32_t tmem_base;
     int abort_flag;
-    std::uint32_t few[2][2][3], flags[2];  // the worst verdicts: whole slabs' and a shorter last slab's, A's and B's
+    std::uint32_t fallback;
 };
 static_assert(sizeof(Barriers) <= 256, "barrier block");
 
@@ -92,7 +93,7 @@ struct Fp16Params {
     std::int64_t c_row_stride, c_col_stride;
     std::int64_t d_row_stride, d_col_stride;
     std::uint32_t m, n;
-    std::uint32_t k_blocks, blocks_per_split, splits;
+    std::uint32_t k, k_blocks, blocks_per_split, splits;
     std::uint32_t tiles_m, tiles_n, tile_n, band_m_tiles;
     std::uint32_t chunk_blocks;
     float alpha, beta;
@@ -100,11 +101,9 @@ struct Fp16Params {
     const float* inverse_a;  // [slab][inverse_pitch_a]
     const float* inverse_b;
     std::uint64_t inverse_pitch_a, inverse_pitch_b;
-    const std::uint32_t* verdicts;  // of the split's CTAs: first A's, then B's
-    std::uint32_t verdicts_a, verdicts_b;
+    const std::uint32_t* verdicts;        // of the split's CTAs: first A's, then B's, slab by slab
+    std::uint32_t verdicts_per_slab[2];
     std::uint32_t slabs;
-    std::uint32_t slabs_fastest;    // bit 0: A's verdicts run through the slabs first (else slab by slab), bit 1: B's
-    std::uint32_t short_slab;       // the last slab is shorter than the others
     std::uint32_t* use_fallback;    // the decision, for the kernels behind this one
     std::uint32_t vector;  // consecutive columns of the output and C that one aligned access takes: 8, 4, or 0 (any strides)
     int* status;
@@ -273,8 +272,7 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         mbarrierInit(&bars->flush_x, 1);
         mbarrierInit(&bars->flush_h, 1);
         bars->abort_flag = 0;
-        for (int i = 0; i < 12; ++i) { bars->few[i / 6][i / 3 % 2][i % 3] = 0; }
-        bars->flags[0] = bars->flags[1] = 0;
+        bars->fallback   = 0;
         fenceBarrierInit();
         prefetchTensorMap(&map_a);
         prefetchTensorMap(&map_b);
@@ -292,48 +290,39 @@ tensorGemm3xFp16(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     gridDependencyLaunchDependents();
     // Every CTA comes to the same decision. Left to the fallback, there are no items.
     {
-        // A gray element only concerns its own slab. A shorter last slab is kept apart from the others: of a handful of K
-        // values a column can well have none of full size, and a gray element elsewhere is no reason to mind.
-        for (int which = 0; which < 2; ++which) {
-            const std::uint32_t* const verdicts = p.verdicts + (which != 0 ? p.verdicts_a : 0);
-            const std::uint32_t count           = which != 0 ? p.verdicts_b : p.verdicts_a;
-            const bool slabs_fastest            = (p.slabs_fastest >> which & 1U) != 0;
-            const std::uint32_t last_slab_at    = count - count / p.slabs;
-            std::uint32_t few[2][3] = {{0, 0, 0}, {0, 0, 0}}, flags[2] = {0, 0};
-#pragma unroll 4
-            for (std::uint32_t i = threadIdx.x; i < count; i += kThreads) {
-                const std::uint32_t verdict = __ldcg(verdicts + i);
-                const bool in_last = p.short_slab != 0 && (slabs_fastest ? i % p.slabs == p.slabs - 1 : i >= last_slab_at);
-                flags[0] |= in_last ? 0U : verdict;
-                flags[1] |= in_last ? verdict : 0U;
+        // A warp takes a slab at a time: a gray element only concerns its own.
+        for (std::uint32_t slab = warp; slab < p.slabs; slab += kThreads / 32) {
+            const std::uint32_t length = min(kSlabK, p.k - slab * kSlabK);
+            std::uint32_t small[2][3]  = {{0, 0, 0}, {0, 0, 0}}, state = fp16x3::kAllCovered;
 #pragma unroll
-                for (int t = 0; t < 3; ++t) {
-                    const std::uint32_t small = verdict >> (10 * t) & fp16x3::kVerdictFew;
-                    few[0][t] = max(few[0][t], in_last ? 0U : small);
-                    few[1][t] = max(few[1][t], in_last ? small : 0U);
+            for (int which = 0; which < 2; ++which) {
+                const std::uint32_t count           = p.verdicts_per_slab[which];
+                const std::uint32_t* const verdicts = p.verdicts + (which != 0 ? p.slabs * p.verdicts_per_slab[0] : 0) + slab * count;
+#pragma unroll 1
+                for (std::uint32_t at = lane; at < count; at += 32 * 8) {
+                    std::uint32_t v[8];
+#pragma unroll
+                    for (std::uint32_t i = 0; i < 8; ++i) { v[i] = at + 32 * i < count ? __ldcg(verdicts + at + 32 * i) : 0; }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        state = max(state, v[i] >> fp16x3::kVerdictState);
+#pragma unroll
+                        for (int t = 0; t < 3; ++t) { small[which][t] = max(small[which][t], v[i] >> (10 * t) & fp16x3::kVerdictSmall); }
+                    }
                 }
+#pragma unroll
+                for (int t = 0; t < 3; ++t) { small[which][t] = __reduce_max_sync(0xFFFFFFFFU, small[which][t]); }
             }
-#pragma unroll
-            for (int kind = 0; kind < 2; ++kind) {
-                flags[kind] = __reduce_or_sync(0xFFFFFFFFU, flags[kind]);
-                if (lane == 0) { atomicOr(&bars->flags[kind], flags[kind]); }
-#pragma unroll
-                for (int t = 0; t < 3; ++t) {
-                    few[kind][t] = __reduce_max_sync(0xFFFFFFFFU, few[kind][t]);
-                    if (lane == 0) { atomicMax(&bars->few[kind][which][t], few[kind][t]); }
-                }
+            state = __reduce_max_sync(0xFFFFFFFFU, state);
+            // F_a + F_b - L >= (g_a + g_b) / 128 for any pair of thresholds whose exponents add up to 18.
+            const std::uint32_t common = state == fp16x3::kManyGray ? (2 * length + 127) / 128 : 1;
+            const auto enough          = [&](int a, int b) { return small[0][a] + small[1][b] + common <= length; };
+            if (state == fp16x3::kOutOfRange || (state != fp16x3::kAllCovered && !enough(0, 2) && !enough(1, 1) && !enough(2, 0))) {
+                if (lane == 0) { bars->fallback = 1; }
             }
         }
         __syncthreads();
-        bool fallback = false;
-#pragma unroll
-        for (int kind = 0; kind < 2; ++kind) {
-            // F_a + F_b - 1 >= 1/64, in 1023rds of a slab and with one to spare for the rounding of each, for any pair
-            // of thresholds whose exponents add up to 18.
-            const auto enough = [&](int a, int b) { return bars->few[kind][0][a] + bars->few[kind][1][b] + 16 + 2 <= 1023; };
-            fallback = fallback || (bars->flags[kind] & fp16x3::kVerdictOutOfRange) != 0 ||
-                       ((bars->flags[kind] & fp16x3::kVerdictGray) != 0 && !enough(0, 2) && !enough(1, 1) && !enough(2, 0));
-        }
+        const bool fallback = bars->fallback != 0;
         if (blockIdx.x == 0 && threadIdx.x == 0) { *p.use_fallback = fallback ? 1U : 0U; }
         if (fallback) { num_items = 0; }
     }
@@ -679,6 +668,7 @@ cudaError_t launchPrepared(const LaunchState& state, void* workspace, cudaStream
     p.d_col_stride     = desc.d_col_stride;
     p.m                = static_cast<std::uint32_t>(desc.m);
     p.n                = static_cast<std::uint32_t>(desc.n);
+    p.k                = split.k;
     p.k_blocks         = split.k_blocks;
     p.blocks_per_split = prepared.blocks_per_split;
     p.splits           = prepared.splits;
@@ -695,11 +685,8 @@ cudaError_t launchPrepared(const LaunchState& state, void* workspace, cudaStream
     p.inverse_pitch_a  = prepared.inverse_pitch[0];
     p.inverse_pitch_b  = prepared.inverse_pitch[1];
     p.verdicts         = verdicts;
-    p.verdicts_a       = split.operand[0].blocks;
-    p.verdicts_b       = split.operand[1].blocks;
     p.slabs            = split.slabs;
-    p.slabs_fastest    = split.operand[0].along_k | split.operand[1].along_k << 1;
-    p.short_slab       = split.k % fp16x3::kSlabK != 0 ? 1U : 0U;
+    for (int i = 0; i < 2; ++i) { p.verdicts_per_slab[i] = split.operand[i].blocks / split.slabs; }
     p.use_fallback     = decision;
     p.status           = state.device_status;
     const auto aligned = [&](std::uint32_t width, const float* at, std::int64_t row_stride, std::int64_t col_stride) {

@@ -8,15 +8,18 @@
 // 2^26 of the largest; below that ("gray" elements) to within 2^-36, which is 2^-50 of the largest.
 //
 // When that is enough. An element's error e contributes e * |b| to the result: for a gray element of A at most
-// 2^-50 M_a M_b, with M the largest magnitude that either scale allows for. If at least F_a elements of every row of A
-// reach 2^-s M_a and F_b of every column of B reach 2^-t M_b, any row and column have F_a + F_b - 768
-// positions where both do, so sum |a||b| over the slab is at least (F_a + F_b - 768) 2^-(s+t) M_a M_b. With
-// s + t = 18 and F_a + F_b - 768 >= 12, all gray elements of both add at most 2 * 768 * 2^-50 against 12 * 2^-18:
+// 2^-50 M_a M_b, with M the largest magnitude that either scale allows for, and with g_a gray elements in a row of A and g_b in
+// a column of B at most (g_a + g_b) 2^-50 M_a M_b in all. If at least F_a elements of every nonzero row of A
+// reach 2^-s M_a and F_b of every nonzero column of B reach 2^-t M_b, any row and column have F_a + F_b - L of the slab's L
+// positions where both do, so sum |a||b| over the slab is at least (F_a + F_b - L) 2^-(s+t) M_a M_b. With
+// s + t = 18 and F_a + F_b - L >= (g_a + g_b) / 128, the gray elements add at most
 // 2^-25 of sum |a||b|, below the rounding of an FP32 product. The elements are counted for s (and t) of 5, 9 and 13, so
-// that an operand with a few very large elements -- outliers of activations -- is made up for by an even one. No gray
-// element at all needs no count. Otherwise, or when a largest magnitude is outside [2^-100, 2^61), infinite or
+// that an operand with a few very large elements -- outliers of activations -- is made up for by an even one; of the gray ones it
+// is only told whether a row has up to 64 of them (two such rows need one position in common) or more (counted as L each). No
+// gray element at all needs no count. All of this concerns one slab: a gray element here is no reason to mind a row that is
+// nearly empty there. Where it is not enough, or a largest magnitude is outside [2^-100, 2^61), infinite or
 // NaN, the launch is left to the TF32 kernel, which splits without scaling. Every CTA leaves a verdict; the
-// multiplying kernel takes the worst of them all.
+// multiplying kernel decides slab by slab and then for the whole launch.
 //
 // The scales belong to slabs, and not to whole rows, so that one pass is enough: a CTA holds a slab of
 // some rows, takes their largest magnitudes, and converts. HBM-bound: 4 bytes read and 4 written an element.
@@ -81,8 +84,11 @@ __device__ __forceinline__ RowScale rowScale(std::uint32_t most) {
     return {__uint_as_float((268 - exponent) << 23), __uint_as_float((exponent - 14) << 23), true};
 }
 
+__device__ __forceinline__ std::uint32_t grayElement(float x, float scale) { return x != 0.0F && fabsf(x * scale) < 0x1p-12F ? 1U : 0U; }
+
 // Splits pairs of elements of one row and keeps what the verdict needs: how many reach each threshold (in the scaled
-// numbers, whose largest is below 2^15), and the smallest nonzero magnitude.
+// numbers, whose largest is below 2^15), and the smallest nonzero magnitude. Gray elements are rare: they are only counted,
+// in another pass over what the CTA still holds, where there are any.
 struct PairSplitter {
     float2 scale;
     __half2 large[3];                  // counts, in halves: at most 2048 each
@@ -127,28 +133,29 @@ __device__ __forceinline__ void worstCounts(std::uint32_t (&worst)[3], std::uint
 __global__ void __launch_bounds__(kThreads, 2) splitOperands(const SplitParams p) {
     extern __shared__ float tile[];
     __shared__ std::uint32_t most_of[kWarps][kSplitRows];
-    __shared__ std::uint32_t large_of[kSplitRows];
+    __shared__ std::uint32_t large_of[kSplitRows], gray_of[kSplitRows];
     __shared__ float scale_of[kSplitRows];
-    __shared__ std::uint32_t worst_of[kWarps][3], flags_of[kWarps];
+    __shared__ std::uint32_t worst_of[kWarps][3], state_of[kWarps];
     const std::uint32_t which = blockIdx.x < p.operand[0].blocks ? 0 : 1;
     const SplitOperand& o     = p.operand[which];
     const std::uint32_t block = blockIdx.x - (which != 0 ? p.operand[0].blocks : 0);
     const std::uint32_t warp  = threadIdx.x >> 5;
     const std::uint32_t lane  = threadIdx.x & 31;
     const std::uint64_t pitch = p.k_blocks * kBlockBytes;
-    bool gray                 = false;
-    bool covered              = true;
+    std::uint32_t state       = kAllCovered;
     std::uint32_t worst[3]    = {0, 0, 0};  // small elements of the worst row this thread knows
     gridDependencyWait();
     gridDependencyLaunchDependents();
-    std::uint32_t slab, row0;
+    const std::uint32_t row_blocks = o.blocks / p.slabs;
+    std::uint32_t slab, row_block, row0;
     if (o.along_k != 0) {  // neighbouring CTAs take neighbouring pieces of memory
-        slab = block % p.slabs;
-        row0 = block / p.slabs * kSplitRowsAlongK;
+        slab      = block % p.slabs;
+        row_block = block / p.slabs;
+        row0      = row_block * kSplitRowsAlongK;
     } else {
-        const std::uint32_t row_blocks = (o.rows + kSplitRows - 1) / kSplitRows;
-        slab = block / row_blocks;
-        row0 = block % row_blocks * kSplitRows;
+        slab      = block / row_blocks;
+        row_block = block % row_blocks;
+        row0      = row_block * kSplitRows;
     }
     const std::uint32_t begin  = slab * kSlabK;
     const std::uint32_t depth  = min(p.k, begin + kSlabK);
@@ -177,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 2) splitOperands(const SplitParams p
             of_group = __reduce_max_sync(0xFFFFFFFFU, large_of[lane % kWarps]);
         }
         const RowScale scaling = rowScale(of_group);
-        covered                = scaling.covered;
+        if (!scaling.covered) { state = kOutOfRange; }
         if (row < o.rows) {
             unsigned char* target = o.split + row * pitch + begin / kBlockK * kBlockBytes + lane / 16 * kBlockBytes + lane % 16 * 8;
             PairSplitter splitter(scaling.scale);
@@ -191,14 +198,23 @@ __global__ void __launch_bounds__(kThreads, 2) splitOperands(const SplitParams p
                     *reinterpret_cast<uint2*>(target + i * 2 * kBlockBytes + 2 * kBlockK) = lo;
                 }
             }
-            gray                      = splitter.sawGray();
+            if (__any_sync(0xFFFFFFFFU, splitter.sawGray())) {
+                std::uint32_t gray = 0;
+#pragma unroll
+                for (std::uint32_t i = 0; i < kSlabK / 128; ++i) {
+                    gray += grayElement(v[i].x, scaling.scale) + grayElement(v[i].y, scaling.scale) +
+                            grayElement(v[i].z, scaling.scale) + grayElement(v[i].w, scaling.scale);
+                }
+                gray  = __reduce_add_sync(0xFFFFFFFFU, gray);
+                state = max(state, gray > kFewGrayElements ? kManyGray : kFewGray);
+            }
             const std::uint32_t large = __reduce_add_sync(0xFFFFFFFFU, splitter.largeElements());
             if (most != 0) { worstCounts(worst, large, length); }
             if (lane == 0) { o.inverse[slab * o.pitch + (o.grouped != 0 ? row / kColumnGroup : row)] = scaling.inverse; }
         }
     } else {
         // The slab is turned in shared memory: read along the rows, written along K.
-        if (threadIdx.x < kSplitRows) { large_of[threadIdx.x] = 0; }
+        if (threadIdx.x < kSplitRows) { large_of[threadIdx.x] = gray_of[threadIdx.x] = 0; }
         if (o.vector != 0) {
             // 16-byte loads: a warp takes 4 K values of all 32 rows.
             const std::uint32_t at_row = lane % 8 * 4;
@@ -275,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, 2) splitOperands(const SplitParams p
             }
             const RowScale scaling  = rowScale(of_group);
             const std::uint32_t row = row0 + threadIdx.x;
-            covered                 = scaling.covered;
+            if (!scaling.covered) { state = kOutOfRange; }
             scale_of[threadIdx.x]   = scaling.scale;
             if (row < o.rows) { o.inverse[slab * o.pitch + (o.grouped != 0 ? row / kColumnGroup : row)] = scaling.inverse; }
         }
@@ -301,33 +317,45 @@ __global__ void __launch_bounds__(kThreads, 2) splitOperands(const SplitParams p
                 *reinterpret_cast<uint4*>(at + 2 * kBlockK) = lo;
             }
         }
-        gray                = splitter.sawGray();
+        if (splitter.sawGray()) {
+            std::uint32_t gray = 0;
+            from               = tile + (first * kBlockK + lane % 8 * 8) * kTilePitch + at_row;
+#pragma unroll 1
+            for (std::uint32_t i = 0; i < kSlabBlocks / 2; ++i, from += kBlockK * kTilePitch) {
+                for (int j = 0; j < 8; ++j) { gray += grayElement(from[j * kTilePitch], scale_of[at_row]); }
+            }
+            atomicAdd(&gray_of[at_row], gray);
+        }
         std::uint32_t large = splitter.largeElements();
         large += __shfl_xor_sync(0xFFFFFFFFU, large, 1);
         large += __shfl_xor_sync(0xFFFFFFFFU, large, 2);
         large += __shfl_xor_sync(0xFFFFFFFFU, large, 4);
         if (lane % 8 == 0) { atomicAdd(&large_of[at_row], large); }
         __syncthreads();
-        if (threadIdx.x < kSplitRows && most != 0) { worstCounts(worst, large_of[threadIdx.x], length); }
+        if (threadIdx.x < kSplitRows && most != 0) {
+            worstCounts(worst, large_of[threadIdx.x], length);
+            const std::uint32_t gray = gray_of[threadIdx.x];
+            if (gray != 0) { state = max(state, gray > kFewGrayElements ? kManyGray : kFewGray); }
+        }
     }
-    const bool any_gray = __any_sync(0xFFFFFFFFU, gray), all_covered = __all_sync(0xFFFFFFFFU, covered);
+    state = __reduce_max_sync(0xFFFFFFFFU, state);
 #pragma unroll
     for (int t = 0; t < 3; ++t) { worst[t] = __reduce_max_sync(0xFFFFFFFFU, worst[t]); }
     if (lane == 0) {
 #pragma unroll
-        for (int t = 0; t < 3; ++t) { worst_of[warp][t] = (worst[t] * 1023 + length - 1) / length; }
-        flags_of[warp] = (any_gray ? kVerdictGray : 0U) | (all_covered ? 0U : kVerdictOutOfRange);
+        for (int t = 0; t < 3; ++t) { worst_of[warp][t] = worst[t]; }
+        state_of[warp] = state;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        std::uint32_t few[3] = {0, 0, 0}, verdict = 0;
+        std::uint32_t small[3] = {0, 0, 0}, worst_state = kAllCovered;
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) {
-            verdict |= flags_of[w];
+            worst_state = max(worst_state, state_of[w]);
 #pragma unroll
-            for (int t = 0; t < 3; ++t) { few[t] = max(few[t], worst_of[w][t]); }
+            for (int t = 0; t < 3; ++t) { small[t] = max(small[t], worst_of[w][t]); }
         }
-        o.verdicts[block] = verdict | few[0] | few[1] << 10 | few[2] << 20;
+        o.verdicts[slab * row_blocks + row_block] = worst_state << kVerdictState | small[0] | small[1] << 10 | small[2] << 20;
     }
 }
 

@@ -145,6 +145,33 @@ def test_a_gray_element_concerns_its_own_slab_only(capi, gpu, oracle, k, transpo
                        run(capi, gpu, capi.KERNEL_TF32X3, a_view, b_view, None, 1.0, 0.0)), "kept the FP16 kernel"
 
 
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("kind", ["other slab", "sparse", "many"])
+def test_sparse_rows_and_gray_elements(capi, gpu, oracle, kind, transposed):
+    """A row with next to nothing in one slab and a tiny element in another slab have nothing to do with each other, and a few
+    tiny elements ask for one position in common only; a row that is tiny but for ten elements asks for more than ten leave."""
+    torch.manual_seed(5)
+    m, k, n = 520, 2000, 900
+    a, b = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda")
+    if kind == "other slab":
+        a[9, 2:768] = 0.0                # slab 0: two elements, fewer than the small ones of a column
+        b[:768] = torch.where(b[:768].abs() < 0.01, 0.01, b[:768])
+        b[0:2, 4] = 2.0 ** -14
+        a[30, 1000] = b[1900, 17] = 2.0 ** -40   # slabs 1 and 2
+    elif kind == "sparse":               # 95 % zeros, tiny elements everywhere
+        a *= torch.rand(m, k, device="cuda") < 0.05
+        a[::7, 100::500] = 2.0 ** -40
+        b[50::300, ::5] = 2.0 ** -40
+    else:
+        a[9, 10:768] *= 2.0 ** -32
+    a_view, b_view = (a.t().contiguous().t(), b.t().contiguous().t()) if transposed else (a, b)
+    for kernel, plain in ((capi.KERNEL_FP16X3, capi.KERNEL_TF32X3), (capi.KERNEL_FP16X3_SPLITK, capi.KERNEL_TF32X3_SPLITK)):
+        d = run(capi, gpu, kernel, a_view, b_view, None, 1.0, 0.0)
+        check(oracle, d, a, b, None, 1.0, 0.0, kind)
+        left = torch.equal(d, run(capi, gpu, plain, a_view, b_view, None, 1.0, 0.0))
+        assert left == (kind == "many"), "went to the TF32 kernel" if left else "kept the FP16 kernel"
+
+
 def test_a_plan_offers_both_forms(capi, gpu, oracle):
     """Index 0 asks for the prepared form's workspace, the same Primitive without it follows, and index 0 still
     runs with less."""
