@@ -15,12 +15,17 @@ std::uint64_t ceilDiv(std::uint64_t x, std::uint64_t y) { return (x + y - 1) / y
 // there is enough work (2048 x 512 x 1024 37 / 29, 1024 x 16384 x 2048 316 / 293, 2048^3 115 / 63, 4096^3 710 / 412,
 // 8192 x 4096 x 8192 2779 / 1438); at 455 and 512 only with a medium K (1024 x 4096 x 1024 59 / 51, 512 x 2048 x 4096 65 / 50,
 // but 1024^3 26 / 27, 512 x 16384 x 4096 326 / 356); below that hardly ever (512 x 4096 x 2048 51 / 60,
-// 256 x 4096 x 4096 50 / 75). A K under 512 was not measured.
+// 256 x 4096 x 4096 50 / 75). Up to 45 tiles of 128 x 192 the TF32 form spreads a K of up to 4096 over clusters of three
+// CTAs or more and needs more work to be overtaken: 33.3 / 40.9 at 1040 x 2184 x 888, 35.1 / 45.3
+// at 830 x 2368 x 1152, 41.2 / 43.8 at 768 x 3264 x 1148, but 49.4 / 47.9 at 904 x 4096 x 904 and, with 48 tiles,
+// 58.4 / 44.0 at 688 x 3456 x 1384. A K under 512 was not measured.
 bool preparedFormPays(const GemmShape& shape) noexcept {
     if (shape.k < 512 || shape.m < 512 || shape.n < 512) { return false; }
     const double m = static_cast<double>(shape.m), n = static_cast<double>(shape.n), products = m * n * static_cast<double>(shape.k);
     const double reuse = m * n / (m + n);
-    return reuse >= 600.0 ? products >= 1e9 : reuse >= 450.0 && products >= 1.5e9 && products <= 6e9;
+    if (reuse >= 600.0) { return products >= 1e9; }
+    const bool few_tiles = ceilDiv(shape.m, 128) * ceilDiv(shape.n, 192) <= 45;
+    return reuse >= 450.0 && products >= (few_tiles ? 3e9 : 1.5e9) && products <= 6e9;
 }
 
 // Regime map on B200 (148 SMs; the count is queried, not assumed). The
