@@ -7,10 +7,11 @@
 
 #include <cstdint>
 
+#include "fp16x3_geometry.hpp"
+
 namespace ftcuda {
 namespace fp16x3 {
 
-constexpr std::uint32_t kBlockK     = 64;   // K elements of one block: 128 bytes of FP16, one swizzle row
 constexpr std::uint32_t kSlabBlocks = 12;   // K blocks with scales of their own
 constexpr std::uint32_t kSlabK      = kSlabBlocks * kBlockK;
 

@@ -52,11 +52,11 @@ namespace {
 
 using fp16x3::kBlockBytes;
 using fp16x3::kBlockK;
+using fp16x3::kMaxTileN;
 using fp16x3::kSlabBlocks;
 using fp16x3::kSlabK;
+using fp16x3::kTileM;
 
-constexpr int kTileM      = 256;  // of a CTA pair
-constexpr int kMaxTileN   = 256;
 constexpr int kStages     = 3;
 constexpr int kThreads    = 384;
 constexpr int kABytes     = 128 * static_cast<int>(kBlockBytes);  // a CTA's A tile: high | low, 16 KiB each
@@ -539,36 +539,6 @@ void describeOperands(const FtcudaGemmDesc& desc, fp16x3::SplitOperand (&operand
     operands[1].grouped    = 1;
 }
 
-// Tile width and K slices. Modelled cost in SM cycles: a K step of 16 is three MMAs of tile_n / 2 cycles each, or the
-// shared-memory traffic behind them (operand fetches and TMA writes at 128 bytes a cycle) where that is longer, which it is
-// under 192 columns; a tile costs about 4000 more (pipeline fill, last drain, output); K slices cost a second
-// kernel and their sums' way through memory.
-struct Geometry {
-    std::uint32_t tile_n, splits, blocks_per_split;
-    double cycles;
-};
-
-Geometry chooseGeometry(std::uint64_t m, std::uint64_t n, std::uint64_t k_blocks, std::uint64_t pairs) {
-    Geometry best{kMaxTileN, 1, static_cast<std::uint32_t>(k_blocks), 0.0};
-    for (std::uint32_t width = kMaxTileN; width >= 64; width -= 16) {
-        const std::uint64_t tiles = ceilDiv(m, kTileM) * ceilDiv(n, width);
-        const double mma          = 1.5 * width;
-        const double smem         = 160.0 + 0.625 * width;
-        const double block_cycles = 4.0 * (mma > smem ? mma : smem);
-        for (std::uint32_t splits = 1; splits <= 32; ++splits) {
-            const std::uint64_t per_split = splits == 1 ? k_blocks : roundUp(ceilDiv(k_blocks, splits), 4);
-            if (splits > 1 && ( ceilDiv(k_blocks, per_split) != splits)) { continue; }
-            if (tiles * splits >= (1ULL << 31)) { break; }
-            double cycles = static_cast<double>(ceilDiv(tiles * splits, pairs)) * (static_cast<double>(per_split) * block_cycles + 4000.0);
-            if (splits > 1) { cycles += 8000.0 + static_cast<double>(m) * static_cast<double>(n) * (8.0 * splits + 4.0) / 3500.0; }
-            if (best.cycles == 0.0 || cycles < best.cycles) {
-                best = Geometry{width, splits, static_cast<std::uint32_t>(per_split), cycles};
-            }
-        }
-    }
-    return best;
-}
-
 }  // namespace
 
 const char* supportsPrepared(const FtcudaGemmDesc& desc) {
@@ -588,7 +558,7 @@ int configurePrepared(LaunchState& state, const FtcudaGemmDesc& desc, char* mess
     prepared.desc           = desc;
     const std::uint64_t k_blocks = ceilDiv(desc.k, kBlockK);
     const std::uint64_t pairs    = static_cast<std::uint64_t>(sms) / 2;
-    const Geometry geometry      = chooseGeometry(desc.m, desc.n, k_blocks, pairs);
+    const fp16x3::Geometry geometry = fp16x3::chooseGeometry(desc.m, desc.n, k_blocks, pairs);
     prepared.tile_n              = geometry.tile_n;
     prepared.splits              = geometry.splits;
     prepared.blocks_per_split    = geometry.blocks_per_split;

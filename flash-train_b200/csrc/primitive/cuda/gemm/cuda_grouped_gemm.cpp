@@ -1,6 +1,5 @@
 #include "primitive/cuda/gemm/cuda_grouped_gemm.hpp"
 
-#include <algorithm>
 #include <cstdint>
 
 #include "cuda/large_group.hpp"
@@ -117,7 +116,9 @@ void CudaGroupedGemm::configure(const GroupedGemmProblem& problem) {
     };
     launch_          = make(kernel_);
     workspace_bytes_ = ftcuda_grouped_gemm_workspace_bytes(launch_.get());
-    if (kernel_ == FTCUDA_GROUPED_GEMM_TF32X3 && std::any_of(descs.begin(), descs.end(), ftcuda::largeGroup) &&
+    std::int32_t sms = 148;
+    if (ftcuda_device_sm_count(getCurrentDeviceId(), &sms, nullptr, 0) != 0 || sms <= 0) { sms = 148; }
+    if (kernel_ == FTCUDA_GROUPED_GEMM_TF32X3 && ftcuda::preparedGroupsPay(descs.data(), count, static_cast<std::uint32_t>(sms)) &&
         ftcuda_grouped_gemm_supports(FTCUDA_GROUPED_GEMM_FP16X3, descs.data(), count, reason, sizeof reason) == 0) {
         prepared_       = make(FTCUDA_GROUPED_GEMM_FP16X3);
         prepared_bytes_ = ftcuda_grouped_gemm_workspace_bytes(prepared_.get());

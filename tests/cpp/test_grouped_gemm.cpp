@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "core/handle.hpp"
+#include "cuda/large_group.hpp"
 #include "fake_platform.hpp"
 #include "family/grouped_gemm/family.hpp"
 #include "flash_train/flash_train.h"
@@ -315,6 +316,22 @@ TEST(grouped_gemm_with_only_empty_groups_plans_and_runs_nothing) {
 
 // GroupedBCDGemm (a is a TensorList) and GroupedABGemm (c and d are TensorLists): a list's g-th view is group g,
 // an ordinary matrix view with its own address, extents and (optional) strides.
+TEST(grouped_prepared_form_where_it_was_measured_to_pay) {
+    const auto pays = [](const std::vector<std::uint64_t>& rows, std::uint64_t k, std::uint64_t n) {
+        std::vector<FtcudaGemmDesc> groups(rows.size(), FtcudaGemmDesc{});
+        for (std::size_t g = 0; g < rows.size(); ++g) { groups[g].m = rows[g], groups[g].n = n, groups[g].k = k; }
+        return ftcuda::preparedGroupsPay(groups.data(), static_cast<std::uint32_t>(groups.size()), 148);
+    };
+    using Rows = std::vector<std::uint64_t>;
+    CHECK(pays({1492, 0, 1117, 1861, 744, 1489, 372, 1117}, 4096, 4096) && pays(Rows(8, 2048), 1024, 2048) && pays(Rows(4, 1500), 2048, 2048));
+    CHECK(pays({1200}, 2816, 1200) && pays({7286, 0}, 1856, 3712) && pays({1500, 130}, 2048, 2048));
+    // Each group alone would be faster in the prepared form; together their tiles fill the waves of the one launch.
+    CHECK(!pays(Rows(4, 1200), 2816, 1200) && !pays(Rows(8, 1100), 4096, 1536) && !pays(Rows(8, 1024), 4096, 1472) && !pays(Rows(8, 1408), 2048, 1408));
+    // The others need a launch of their own, where there was room for them in the large group's last wave.
+    CHECK(!pays({1500, 130}, 2048, 1536) && !pays({1500, 100, 100, 100}, 2048, 1536));
+    CHECK(!pays({}, 2048, 2048) && !pays({0, 0}, 2048, 2048) && !pays(Rows(16, 512), 2048, 2048));
+}
+
 TEST(grouped_problem_takes_tensor_lists) {
     Ragged ragged;
     const std::int64_t dims[3][2]  = {{256, 512}, {0, 512}, {130, 260}};
