@@ -82,7 +82,6 @@ extern "C" int ftcuda_gemm_configure(int kernel, const FtcudaGemmDesc* desc, Ftc
     if (reason != nullptr) { return ftcuda::fail(message, message_capacity, 1, "%s", reason); }
     std::memset(launch, 0, sizeof *launch);
     LaunchState& state  = *reinterpret_cast<LaunchState*>(launch);
-    const int requested = kernel;
     const bool prepared = fallbackOf(kernel) >= 0;
     if (prepared) { kernel = fallbackOf(kernel); }
     state.desc   = *desc;
@@ -105,11 +104,23 @@ extern "C" int ftcuda_gemm_configure(int kernel, const FtcudaGemmDesc* desc, Ftc
         state.stage_bytes += 256;
         state.workspace_bytes += state.stage_bytes;
     }
-    if (status == 0 && prepared) {
-        status                         = ftcuda::configurePrepared(state, *desc, message, message_capacity);
-        state.prepared.fallback_kernel = kernel;
-        state.kernel                   = requested;
+    if (status == 0 && prepared) { status = ftcuda_gemm_prepare(launch, desc, launch, message, message_capacity); }
+    return status;
+}
+
+extern "C" int ftcuda_gemm_prepare(const FtcudaGemmLaunch* launch, const FtcudaGemmDesc* desc, FtcudaGemmLaunch* prepared, char* message,
+                                   size_t message_capacity) {
+    if (launch == nullptr || desc == nullptr || prepared == nullptr) { return ftcuda::fail(message, message_capacity, 1, "null argument"); }
+    const int kernel = reinterpret_cast<const LaunchState*>(launch)->kernel;
+    if (kernel != FTCUDA_GEMM_TF32X3 && kernel != FTCUDA_GEMM_TF32X3_SPLITK) {
+        return ftcuda::fail(message, message_capacity, 1, "the kernel family has no prepared form");
     }
+    if (const char* reason = ftcuda::supportsPrepared(*desc)) { return ftcuda::fail(message, message_capacity, 1, "%s", reason); }
+    if (prepared != launch) { *prepared = *launch; }
+    LaunchState& state = *reinterpret_cast<LaunchState*>(prepared);
+    const int status   = ftcuda::configurePrepared(state, *desc, message, message_capacity);
+    state.prepared.fallback_kernel = kernel;
+    state.kernel                   = kernel == FTCUDA_GEMM_TF32X3 ? FTCUDA_GEMM_FP16X3 : FTCUDA_GEMM_FP16X3_SPLITK;
     return status;
 }
 

@@ -15,15 +15,6 @@ constexpr GemmPort kAllPorts[]    = {GemmPort::kA, GemmPort::kB,     GemmPort::k
                                      GemmPort::kD, GemmPort::kAlpha, GemmPort::kBeta};
 constexpr GemmPort kMatrixPorts[] = {GemmPort::kA, GemmPort::kB, GemmPort::kC, GemmPort::kD};
 
-// The prepared form of a kernel family, or -1.
-int preparedForm(int kernel) noexcept {
-    switch (kernel) {
-        case FTCUDA_GEMM_TF32X3: return FTCUDA_GEMM_FP16X3;
-        case FTCUDA_GEMM_TF32X3_SPLITK: return FTCUDA_GEMM_FP16X3_SPLITK;
-        default: return -1;
-    }
-}
-
 }  // namespace
 
 const char* cudaGemmName(int kernel) noexcept {
@@ -121,11 +112,8 @@ void CudaGemm::configure(const GemmProblem& problem) {
         throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "%s: configuring the launch failed: %s", getName(), reason);
     }
     workspace_bytes_ = ftcuda_gemm_workspace_bytes(&launch_);
-    const int prepared = preparedForm(kernel_);
-    if (prepared >= 0 && preparedFormPays(problem.getShape()) && ftcuda_gemm_supports(prepared, &desc, reason, sizeof reason) == 0) {
-        if (ftcuda_gemm_configure(prepared, &desc, &prepared_, reason, sizeof reason) != 0) {
-            throw Exception(FTRAIN_STATUS_INTERNAL_ERROR, "%s: configuring the launch failed: %s", getName(), reason);
-        }
+    const bool tensor = kernel_ == FTCUDA_GEMM_TF32X3 || kernel_ == FTCUDA_GEMM_TF32X3_SPLITK;
+    if (tensor && preparedFormPays(problem.getShape()) && ftcuda_gemm_prepare(&launch_, &desc, &prepared_, reason, sizeof reason) == 0) {
         prepared_bytes_ = ftcuda_gemm_workspace_bytes(&prepared_);
     }
 }

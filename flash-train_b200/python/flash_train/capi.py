@@ -48,7 +48,7 @@ EXPORTED_SYMBOLS = (
 ).split()
 
 PLATFORM_SYMBOLS = (
-    "ftcuda_current_device ftcuda_device_sm_count ftcuda_gemm_supports ftcuda_gemm_configure "
+    "ftcuda_current_device ftcuda_device_sm_count ftcuda_gemm_supports ftcuda_gemm_configure ftcuda_gemm_prepare "
     "ftcuda_gemm_workspace_bytes ftcuda_gemm_launch ftcuda_launch_count ftcuda_trace_push ftcuda_trace_pop "
     "ftcuda_trace_mark ftcuda_gemm_splitk_static ftcuda_gemm_splitk_static_capacity ftcuda_gemm_launch_scatter "
     "ftcuda_device_status ftcuda_device_status_reset ftcuda_selftest_bounded_wait ftcuda_measure_ffma_tflops "

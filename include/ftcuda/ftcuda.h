@@ -100,6 +100,14 @@ FTCUDA_API int ftcuda_gemm_supports(int kernel, const FtcudaGemmDesc* desc, char
 FTCUDA_API int ftcuda_gemm_configure(int kernel, const FtcudaGemmDesc* desc, FtcudaGemmLaunch* launch, char* message,
                                      size_t message_capacity);
 
+/*
+ * The prepared form of a configured launch: `launch` was configured for FTCUDA_GEMM_TF32X3 or FTCUDA_GEMM_TF32X3_SPLITK and
+ * `desc`; `prepared` becomes what ftcuda_gemm_configure makes of the family's prepared form, with `launch` as the
+ * one behind it. Returns 0, or nonzero with a reason in `message` where the family or the problem has no prepared form.
+ */
+FTCUDA_API int ftcuda_gemm_prepare(const FtcudaGemmLaunch* launch, const FtcudaGemmDesc* desc, FtcudaGemmLaunch* prepared,
+                                   char* message, size_t message_capacity);
+
 /* Workspace a configured launch needs, in bytes. */
 FTCUDA_API uint64_t ftcuda_gemm_workspace_bytes(const FtcudaGemmLaunch* launch);
 

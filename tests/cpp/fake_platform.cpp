@@ -87,6 +87,22 @@ extern "C" int ftcuda_gemm_configure(int kernel, const FtcudaGemmDesc* desc, Ftc
     return 0;
 }
 
+// The prepared form of a tensor-core launch: the same blob with the family and the workspace of its prepared form.
+extern "C" int ftcuda_gemm_prepare(const FtcudaGemmLaunch* launch, const FtcudaGemmDesc* desc, FtcudaGemmLaunch* prepared, char* message,
+                                   size_t capacity) {
+    ++fake::state().prepares;
+    *prepared  = *launch;
+    auto* blob = reinterpret_cast<fake::Blob*>(prepared);
+    blob->desc = *desc;
+    switch (blob->kernel) {
+        case FTCUDA_GEMM_TF32X3: blob->kernel = FTCUDA_GEMM_FP16X3; break;
+        case FTCUDA_GEMM_TF32X3_SPLITK: blob->kernel = FTCUDA_GEMM_FP16X3_SPLITK; break;
+        default: return fake::fail(message, capacity, "the kernel family has no prepared form");
+    }
+    blob->workspace += fake::state().prepared_workspace;
+    return fake::state().prepared_workspace != 0 ? 0 : fake::fail(message, capacity, "no prepared form");
+}
+
 extern "C" uint64_t ftcuda_gemm_workspace_bytes(const FtcudaGemmLaunch* launch) {
     return reinterpret_cast<const fake::Blob*>(launch)->workspace;
 }

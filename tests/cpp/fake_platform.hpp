@@ -34,12 +34,14 @@ struct State {
     bool device_query_fails  = false;
     int sm_count             = 148;
     std::uint64_t split_k_workspace = 4096;  // what the fake split-K kernels ask for
+    std::uint64_t prepared_workspace = 0;     // what the prepared forms ask for on top; 0: there are none
     std::vector<LaunchRecord> launches;
     std::vector<GroupedLaunchRecord> grouped_launches;
     std::uint64_t grouped_tensor_workspace = 1024;  // what the fake grouped tensor-core kernel asks for
     int grouped_live = 0;                           // configured grouped launches not yet destroyed
     int configures = 0;
     int supports   = 0;
+    int prepares   = 0;
     // Host-side failure injection: the next configure / launch call answers with this reason (and
     // clears it), the way the real layer reports a failed cudaFuncSetAttribute or kernel launch.
     const char* fail_next_configure = nullptr;

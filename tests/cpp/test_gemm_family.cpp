@@ -230,6 +230,20 @@ TEST(plan_dispatches_only_the_indexed_primitive) {
     fake::reset();
 }
 
+TEST(plan_dispatches_prepared_form_made_from_the_configured_launch) {
+    fake::reset();
+    fake::state().prepared_workspace = 10000;
+    CudaGemm primitive(FTCUDA_GEMM_TF32X3_SPLITK);
+    primitive.configure(problem(2048, 2048, 2048));
+    CHECK_EQ(fake::state().configures, 1);  // the family is laid out once, the prepared form on top of it
+    CHECK_EQ(fake::state().prepares, 1);
+    CHECK_EQ(primitive.getRequiredWorkspaceBytes(), std::uint64_t{14096});
+    primitive.configure(problem(1024, 1024, 1024));  // where it does not pay, nothing is asked of the platform
+    CHECK_EQ(fake::state().prepares, 1);
+    CHECK_EQ(primitive.getRequiredWorkspaceBytes(), std::uint64_t{4096});
+    fake::reset();
+}
+
 TEST(finder_regime_map) {
     fake::reset();
     const Constraints device0{0};
