@@ -1,5 +1,7 @@
 #include "fake_platform.hpp"
 
+#include "cuda/large_group.hpp"
+
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -129,14 +131,18 @@ extern "C" int ftcuda_grouped_gemm_supports(int kernel, const FtcudaGemmDesc* gr
                                             size_t capacity) {
     ++fake::state().supports;
     if (kernel == FTCUDA_GROUPED_GEMM_EXACT) { return 0; }
-    if (kernel != FTCUDA_GROUPED_GEMM_TF32X3) { return fake::fail(message, capacity, "unknown grouped kernel family"); }
-    bool any = false;
+    if (kernel != FTCUDA_GROUPED_GEMM_TF32X3 && kernel != FTCUDA_GROUPED_GEMM_FP16X3) {
+        return fake::fail(message, capacity, "unknown grouped kernel family");
+    }
+    bool any = false, large = kernel == FTCUDA_GROUPED_GEMM_TF32X3;
     for (uint32_t g = 0; g < num_groups; ++g) {
         if (groups[g].m * groups[g].n == 0) { continue; }
         any = true;
         if (ftcuda_gemm_supports(FTCUDA_GEMM_TF32X3, &groups[g], message, capacity) != 0) { return 1; }
         if (groups[g].k < 128) { return fake::fail(message, capacity, "K is too short for the split-precision kernel (under 128)"); }
+        large = large || ftcuda::largeGroup(groups[g]);
     }
+    if (!large) { return fake::fail(message, capacity, "no group is large enough for the prepared form"); }
     return any ? 0 : fake::fail(message, capacity, "every group is empty");
 }
 
@@ -149,7 +155,8 @@ extern "C" int ftcuda_grouped_gemm_configure(int kernel, const FtcudaGemmDesc* g
     }
     auto* made      = new FtcudaGroupedGemmLaunch{};
     made->kernel    = kernel;
-    made->workspace = kernel == FTCUDA_GROUPED_GEMM_TF32X3 ? fake::state().grouped_tensor_workspace : 0;
+    made->workspace = kernel == FTCUDA_GROUPED_GEMM_EXACT ? 0 : fake::state().grouped_tensor_workspace;
+    if (kernel == FTCUDA_GROUPED_GEMM_FP16X3) { made->workspace += fake::state().prepared_workspace; }
     made->groups.assign(groups, groups + num_groups);
     ++fake::state().grouped_live;
     *launch = made;

@@ -255,6 +255,81 @@ TEST(one_shot_gemm_walks_the_workspace_budget) {
     fake::reset();
 }
 
+// Where the prepared form pays, each tensor-core Primitive stands in the Plan twice: with its workspace, and kept to what the
+// family cannot do without. An index runs the prepared form only with all it asks for, the TF32 form with less, and is refused
+// below the minimum.
+TEST(one_shot_and_staged_calls_choose_the_prepared_form_by_workspace) {
+    fake::reset();
+    fake::state().prepared_workspace = 1 << 20;
+    const std::int64_t dims[2] = {2048, 2048};
+    float alpha = 1.0F, beta = 0.0F;
+    GemmGraph g = makeGraph();
+    FTrainOps ops   = nullptr;
+    FTrainArgs args = nullptr;
+    FTrainPlan plan = nullptr;
+    ftrainOpsCreate(&ops, g.pattern);
+    ftrainArgsCreate(&args, ops);
+    ftrainArgsSetTensor(args, g.a, matrix(address(0x10000), dims));
+    ftrainArgsSetTensor(args, g.b, matrix(address(0x20000), dims));
+    ftrainArgsSetTensor(args, g.c, matrix(nullptr, dims));
+    ftrainArgsSetTensor(args, g.d, matrix(address(0x40000), dims));
+    ftrainArgsSetTensor(args, g.alpha, scalar(&alpha));
+    ftrainArgsSetTensor(args, g.beta, scalar(&beta));
+    ftrainArgsSetGemm(args, g.op, FTRAIN_NUMERIC_TYPE_FP32);
+    CHECK_EQ(static_cast<int>(ftrainPlanCreate(&plan, args)), 0);
+
+    const struct {
+        const char* name;
+        std::uint64_t bytes;
+    } expected[] = {{"Fp32Gemm3xTf32SplitK", (1 << 20) + 4096}, {"Fp32Gemm3xTf32SplitK", 4096}, {"Fp32Gemm3xTf32", 1 << 20},
+                    {"Fp32Gemm3xTf32", 0}, {"Fp32GemmSplitK", 4096}, {"Fp32Gemm", 0}};
+    std::uint64_t count = 0, bytes = 0;
+    ftrainPlanGetNumPrimitives(plan, &count);
+    CHECK_EQ(count, std::uint64_t{6});
+    for (std::uint64_t i = 0; i < count && i < 6; ++i) {
+        const char* name = nullptr;
+        ftrainPlanGetPrimitiveName(plan, i, &name);
+        ftrainPlanGetPrimitiveRequiredWorkspaceBytes(plan, i, &bytes);
+        CHECK_EQ(std::string(name), std::string(expected[i].name));
+        CHECK_EQ(bytes, expected[i].bytes);
+    }
+    char buffer[8];
+    const auto runs = [&](std::uint64_t index, void* workspace, std::uint64_t size, int kernel) {
+        const std::size_t before = fake::state().launches.size();
+        CHECK_EQ(static_cast<int>(ftrainPlanExecutePrimitive(plan, index, workspace, size, nullptr)), 0);
+        CHECK_EQ(fake::state().launches.size(), before + 1);
+        CHECK_EQ(fake::state().launches.back().kernel, kernel);
+    };
+    runs(0, buffer, (1 << 20) + 4096, FTCUDA_GEMM_FP16X3_SPLITK);
+    runs(0, buffer, (1 << 20) + 4095, FTCUDA_GEMM_TF32X3_SPLITK);
+    runs(0, buffer, 4096, FTCUDA_GEMM_TF32X3_SPLITK);
+    runs(1, buffer, 1 << 30, FTCUDA_GEMM_TF32X3_SPLITK);  // kept to the minimum, whatever it is given
+    runs(2, buffer, 1 << 20, FTCUDA_GEMM_FP16X3);
+    runs(2, buffer, (1 << 20) - 1, FTCUDA_GEMM_TF32X3);
+    runs(2, nullptr, 0, FTCUDA_GEMM_TF32X3);
+    runs(2, nullptr, 1 << 20, FTCUDA_GEMM_TF32X3);  // no address: no workspace
+    const std::size_t launched = fake::state().launches.size();
+    CHECK_EQ(static_cast<int>(ftrainPlanExecutePrimitive(plan, 0, buffer, 4095, nullptr)), static_cast<int>(FTRAIN_STATUS_INVALID_ARGUMENT));
+    CHECK_EQ(static_cast<int>(ftrainPlanExecutePrimitive(plan, 0, nullptr, 1 << 30, nullptr)), static_cast<int>(FTRAIN_STATUS_INVALID_ARGUMENT));
+    CHECK_EQ(fake::state().launches.size(), launched);
+
+    const auto call = [&](void* workspace, std::uint64_t size) {
+        CHECK_EQ(static_cast<int>(ftrainGemm(matrix(address(0x10000), dims), matrix(address(0x20000), dims), matrix(nullptr, dims),
+                                             matrix(address(0x40000), dims), scalar(&alpha), scalar(&beta), FTRAIN_NUMERIC_TYPE_FP32,
+                                             workspace, size, nullptr)), 0);
+        return fake::state().launches.back().kernel;
+    };
+    CHECK_EQ(call(nullptr, 0), static_cast<int>(FTCUDA_GEMM_TF32X3));
+    CHECK_EQ(call(buffer, (1 << 20) + 4096), static_cast<int>(FTCUDA_GEMM_FP16X3_SPLITK));
+    CHECK_EQ(call(buffer, 1 << 20), static_cast<int>(FTCUDA_GEMM_TF32X3_SPLITK));  // the first index that fits
+    CHECK_EQ(call(buffer, 4095), static_cast<int>(FTCUDA_GEMM_TF32X3));
+    ftrainPlanDestroy(plan);
+    ftrainArgsDestroy(args);
+    ftrainOpsDestroy(ops);
+    ftrainPatternDestroy(g.pattern);
+    fake::reset();
+}
+
 // A failed kernel launch or a failed launch configuration surfaces as INTERNAL_ERROR with the platform's
 // reason in the message (the reference maps hipGetLastError the same way,
 // src/primitive/hygon/gemm/fp32_gemm.hip:47-50, through the catch-all of src/include/flash_train/api.hpp:36-62);

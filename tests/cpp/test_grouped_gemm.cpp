@@ -316,6 +316,42 @@ TEST(grouped_gemm_with_only_empty_groups_plans_and_runs_nothing) {
 
 // GroupedBCDGemm (a is a TensorList) and GroupedABGemm (c and d are TensorLists): a list's g-th view is group g,
 // an ordinary matrix view with its own address, extents and (optional) strides.
+TEST(grouped_plan_dispatches_the_prepared_form_by_workspace) {
+    fake::reset();
+    fake::state().prepared_workspace = 5000;
+    // Two large groups and an empty one.
+    const GroupedSpec a{address(0x10000000), {2048, 0, 2048}, {2048, 2048, 2048}}, b{address(0x20000000), {2048, 2048, 2048}, {2048, 2048, 2048}},
+        c{address(0x30000000), {2048, 0, 2048}, {2048, 2048, 2048}}, d{address(0x40000000), {2048, 0, 2048}, {2048, 2048, 2048}};
+    const GroupedGemmProblem problem(OperandValue(grouped(a)), OperandValue(grouped(b)), OperandValue(grouped(c)), OperandValue(grouped(d)),
+                                     scalar(&g_alpha), scalar(&g_beta), FTRAIN_NUMERIC_TYPE_FP32);
+    char workspace[8];
+    {
+        CudaGroupedGemm primitive(FTCUDA_GROUPED_GEMM_TF32X3);
+        primitive.configure(problem);
+        CHECK_EQ(primitive.getRequiredWorkspaceBytes(), std::uint64_t{6024});
+        CHECK_EQ(primitive.getMinimumWorkspaceBytes(), std::uint64_t{1024});
+        const std::unique_ptr<PrimitiveBase> lean = primitive.cloneForMinimumWorkspace();
+        CHECK(lean != nullptr && lean->getRequiredWorkspaceBytes() == 1024 && lean->cloneForMinimumWorkspace() == nullptr);
+        const auto runs = [&](PrimitiveBase& which, std::uint64_t bytes) {
+            which.execute(Resources{workspace, bytes, nullptr});
+            return fake::state().grouped_launches.back().kernel;
+        };
+        CHECK_EQ(runs(primitive, 6024), static_cast<int>(FTCUDA_GROUPED_GEMM_FP16X3));
+        CHECK_EQ(runs(primitive, 6023), static_cast<int>(FTCUDA_GROUPED_GEMM_TF32X3));
+        CHECK_EQ(runs(*lean, 1 << 30), static_cast<int>(FTCUDA_GROUPED_GEMM_TF32X3));
+        CHECK_THROWS_STATUS(primitive.execute(Resources{workspace, 1023, nullptr}), FTRAIN_STATUS_INVALID_ARGUMENT);
+        CHECK_THROWS_STATUS(primitive.execute(Resources{nullptr, 6024, nullptr}), FTRAIN_STATUS_INVALID_ARGUMENT);
+        primitive.configure(Ragged().problem());  // small groups: no prepared form left over from before
+        CHECK_EQ(primitive.getRequiredWorkspaceBytes(), std::uint64_t{1024});
+        CHECK(primitive.cloneForMinimumWorkspace() == nullptr);
+        CudaGroupedGemm exact(FTCUDA_GROUPED_GEMM_EXACT);
+        exact.configure(problem);
+        CHECK_EQ(exact.getRequiredWorkspaceBytes(), std::uint64_t{0});
+    }
+    CHECK_EQ(fake::state().grouped_live, 0);
+    fake::reset();
+}
+
 TEST(grouped_prepared_form_where_it_was_measured_to_pay) {
     const auto pays = [](const std::vector<std::uint64_t>& rows, std::uint64_t k, std::uint64_t n) {
         std::vector<FtcudaGemmDesc> groups(rows.size(), FtcudaGemmDesc{});

@@ -65,7 +65,8 @@ def test_shapes_and_layouts(capi, gpu, oracle, m, k, n):
 
 
 def test_scales_of_rows_and_columns(capi, gpu, oracle):
-    """Rows of A and columns of B of very different size, and rows without a single nonzero."""
+    """Rows of A and columns of B of very different size, and rows without a single nonzero. (Neighbouring columns that far
+    apart share a scale, so this goes to the TF32 kernel; the test below stays in the FP16 one.)"""
     torch.manual_seed(1)
     m, k, n = 300, 700, 270
     a = torch.randn(m, k, device="cuda") * torch.exp2(torch.randint(-40, 40, (m, 1), device="cuda").float())
@@ -75,6 +76,26 @@ def test_scales_of_rows_and_columns(capi, gpu, oracle):
     exact = a.double() @ b.double()
     bound = (a.double().norm(dim=1, keepdim=True) * b.double().norm(dim=0, keepdim=True)) * 2.0 ** -22
     assert ((d.double() - exact).abs() <= bound).all() and (d[7] == 0).all() and (d[:, 11] == 0).all()
+
+
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("m,k,n", [(300, 1700, 285), (129, 5000, 130)])  # three slabs; K slices that begin inside a slab
+def test_scales_of_slabs_rows_and_column_groups(capi, gpu, m, k, n, transposed):
+    """Every row of A, and every 16 columns of B, of another size in every slab of 768, columns of a group up to 2^8 apart: the
+    FP16 kernel itself has to find each scale. A scale taken from another row, group or slab is wrong by powers of two; the
+    bound is that of 48 truncating additions in a row (2^-23 each) and a few roundings, of the sum of magnitudes."""
+    torch.manual_seed(m)
+    a, b = torch.randn(m, k, device="cuda"), torch.randn(k, n, device="cuda")
+    b *= torch.exp2(torch.randint(-8, 1, (1, n), device="cuda").float())
+    for first in range(0, k, 768):
+        slab = slice(first, first + 768)
+        a[:, slab] *= torch.exp2(torch.randint(-30, 30, (m, 1), device="cuda").float())
+        b[slab] *= torch.exp2(torch.randint(-30, 30, (1, -(-n // 16)), device="cuda").float()).repeat_interleave(16, dim=1)[:, :n]
+    a_view, b_view = (a.t().contiguous().t(), b.t().contiguous().t()) if transposed else (a, b)
+    d = run(capi, gpu, capi.KERNEL_FP16X3, a_view, b_view, None, 1.0, 0.0)
+    bound = 2.0 ** -17 * (a.double().abs() @ b.double().abs())
+    assert ((d.double() - a.double() @ b.double()).abs() <= bound).all()
+    assert not torch.equal(d, run(capi, gpu, capi.KERNEL_TF32X3, a_view, b_view, None, 1.0, 0.0)), "went to the TF32 kernel"
 
 
 @pytest.mark.parametrize("exponent_a,exponent_b", [(-55, -55), (-57, -57), (-63, -63), (-90, -30), (-30, -90), (-98, 55)])
@@ -216,3 +237,20 @@ def test_grouped_plan_mixes_both_forms(capi, gpu, oracle):
             first += m
             if m != 0:
                 check(oracle, d[part], a[part], b[g * k:(g + 1) * k], c[part], 1.5, 0.5, f"group {g}, index {index}, {size} bytes")
+
+
+def test_grouped_plan_of_large_groups_only(capi, gpu, oracle):
+    """Nothing is left for the one TF32 launch."""
+    torch.manual_seed(6)
+    rows, k, n = [2048, 2000], 1024, 2048
+    a, b = torch.randn(sum(rows), k, device="cuda"), torch.randn(2 * k, n, device="cuda")
+    d = torch.full((sum(rows), n), float("nan"), device="cuda")
+    plan = capi.GroupedGemmBinding().make_plan(
+        {"address": a.data_ptr(), "rows": rows, "cols": [k] * 2}, {"address": b.data_ptr(), "rows": [k] * 2, "cols": [n] * 2},
+        {"address": 0, "rows": rows, "cols": [n] * 2}, {"address": d.data_ptr(), "rows": rows, "cols": [n] * 2}, 1.0, 0.0)
+    names = plan.primitive_names()
+    assert names[0] == names[1] and plan.workspace_bytes(0) > plan.workspace_bytes(1)
+    gpu.run_plan(plan, 0)
+    torch.cuda.synchronize()
+    check(oracle, d[:rows[0]], a[:rows[0]], b[:k], None, 1.0, 0.0, "first group")
+    check(oracle, d[rows[0]:], a[rows[0]:], b[k:], None, 1.0, 0.0, "second group")
