@@ -412,11 +412,12 @@ def torch_gemm_overhead(ft_torch, torch, device) -> dict:
 
 # --------------------------------------------------------------------------- ride-along records
 
-def tensor_divisor(names, index) -> int:
-    """How many times the measured BF16 rate exceeds the FP32-product rate of a Plan's tensor-core Primitive: three FP16
-    products in the prepared form (the Plan lists the same Primitive without its workspace right behind it), three TF32
-    products at half the rate otherwise."""
-    prepared = "3xTf32" in names[index] and index + 1 < len(names) and names[index + 1] == names[index]
+def tensor_divisor(plan, index) -> int:
+    """How many times the measured BF16 rate exceeds the FP32-product rate of what a Plan runs at `index` with all the workspace it
+    asks for there: three FP16 products in the prepared form, which is where the same Primitive follows and asks for less;
+    three TF32 products at half the rate otherwise."""
+    prepared = (index + 1 < plan.num_primitives and plan.primitive_name(index + 1) == plan.primitive_name(index)
+                and plan.workspace_bytes(index) > plan.workspace_bytes(index + 1))
     return 3 if prepared else 6
 
 
@@ -511,8 +512,8 @@ def config_records(torch, capi, device, peaks, ffma_tflops) -> dict:
             ("config2_4096_cubed_addend_3xtf32", "Fp32Gemm3xTf32", "tensor", None, None)):
         runner = PlanRunner(torch, a, b, c, d, 1.5, 0.5, primitive)
         if peak is None and bound == "tensor":
-            peak   = peaks["bf16_tflops"] / tensor_divisor(runner.names, runner.index)
-            source = f"{peaks['source']} bf16_tflops / {tensor_divisor(runner.names, runner.index)}"
+            divisor = tensor_divisor(runner.plan, runner.index)
+            peak, source = peaks["bf16_tflops"] / divisor, f"{peaks['source']} bf16_tflops / {divisor}"
         stats = measure_calls(torch, runner.run)
         tflops = flops / (stats["median_us"] * 1e-6) / 1e12
         records[label] = {"primitive": runner.name, **stats, "tflops": round(tflops, 2), "bound": bound,
@@ -552,7 +553,7 @@ def config_records(torch, capi, device, peaks, ffma_tflops) -> dict:
             runner = PlanRunner(torch, a, copies[0], None, d)
             stats = measure_calls(torch, runner.run)
             tflops = 2.0 * m * 4096 * 4096 / (stats["median_us"] * 1e-6) / 1e12
-            divisor = tensor_divisor(runner.names, runner.index)
+            divisor = tensor_divisor(runner.plan, runner.index)
             records[f"config3_{m}x4096x4096_{label}"] = {
                 "primitive": runner.name, "workspace_bytes": runner.size, **stats, "bound": "tensor", "tflops": round(tflops, 2),
                 "frac": round(tflops / (peaks["bf16_tflops"] / divisor), 4), "peak_source": f"{peaks['source']} bf16_tflops / {divisor}"}
@@ -584,7 +585,7 @@ def config_records(torch, capi, device, peaks, ffma_tflops) -> dict:
         stats = measure_calls(torch, call)
         tflops = grouped_flops / (stats["median_us"] * 1e-6) / 1e12
         names = grouped_plan.primitive_names()
-        peak, bound = (peaks["bf16_tflops"] / tensor_divisor(names, index), "tensor") if "3xTf32" in name else (ffma_tflops, "fp32")
+        peak, bound = (peaks["bf16_tflops"] / tensor_divisor(grouped_plan, index), "tensor") if "3xTf32" in name else (ffma_tflops, "fp32")
         grouped[name + ("_without_its_workspace" if index and names[index - 1] == name else "")] = {**stats, "tflops": round(tflops, 2), "bound": bound, "frac": round(tflops / peak, 4) if peak else None,
                          "workspace_bytes": size}
     # The same products as separate Plans of the plain Gemm, one launch each, for comparison.
@@ -726,7 +727,8 @@ def k_split_records(torch, capi, world, rank, device, steps: int, peaks) -> dict
                                 "reduce_scatter_ms": collective_ms, "collective_share": collective_ms / step_ms,
                                 "timed": "whole step, local GEMM alone and reduce_scatter_tensor alone, each in its own event-timed loop "
                                          "(maximum over ranks); the loops run one after another, so clocks under the power cap differ a little",
-                                "frac_of_burst_tensor_peak_per_gpu": flops / (step_ms * 1e-3) / 1e12 / world / (peaks["bf16_tflops"] / 3.0),
+                                "frac_of_burst_tensor_peak_per_gpu": flops / (step_ms * 1e-3) / 1e12 / world /
+                                                                     (peaks["bf16_tflops"] / tensor_divisor(*gemm.local_gemm.last)),
                                 **parity(out)}
     try:
         os.environ.setdefault("TORCH_SYMM_MEM_DISABLE_MULTICAST", "1")  # plain peer mappings, no NVLink multicast object
@@ -930,8 +932,8 @@ def run_k_split(options, torch, capi, world, rank, local_rank, device) -> int:
         ms_per_step = elapsed_ms / options.steps
         value = 2.0 * m * n * k / (ms_per_step * 1e-3) / 1e12
         peaks = measured_peaks()
-        # The local Plan runs the prepared form (three FP16 products), the adding launch the TF32 one.
-        divisor = 6 if distributed and options.workload == KSPLIT_FUSED_WORKLOAD else 3
+        # The launch that adds into the owners' rows is the TF32 form; otherwise it is what the local Plan ran.
+        divisor = 6 if distributed and options.workload == KSPLIT_FUSED_WORKLOAD else tensor_divisor(*gemm.local_gemm.last)
         tensor_peak = peaks["bf16_tflops"] / divisor
         line = {
             "metric": "fp32_gemm_tflops", "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": options.steps,
@@ -1011,7 +1013,7 @@ def main() -> int:
     pointer = workspace.data_ptr() if size else 0
     stream = torch.cuda.current_stream().cuda_stream
 
-    plan_names, with_c = plan.primitive_names(), c is not None
+    plan_names, divisor, with_c = plan.primitive_names(), tensor_divisor(plan, index), c is not None
 
     def step():
         plan.execute(index, pointer, size, stream)
@@ -1142,7 +1144,6 @@ def main() -> int:
                 ffma_tflops = max(ffma_tflops or 0.0, capi.measure_ffma_tflops(local_rank))
         ffma_clocks = ffma_sampler.summary()
     if tensor_kernel:
-        divisor = tensor_divisor(plan_names, index)
         burst_peak = peaks["bf16_tflops"] / divisor
         # The captures are of the TF32 kernel.
         traffic = MEASURED_DRAM_TRAFFIC.get((options.workload, primitive, world)) if divisor == 6 else None

@@ -67,6 +67,7 @@ class _LibraryGemm:
         self._binding = capi.GemmBinding()
         self._plans = {}
         self._refused_bytes, self._refused_calls = 0, 0
+        self.last = None  # (Plan, index) of the latest call
 
     def _workspace(self, sizes, device):
         """(index, workspace) of the first primitive whose workspace torch's allocator can give: the best form of a
@@ -108,6 +109,7 @@ class _LibraryGemm:
         plan, sizes = entry
         index, workspace = self._workspace(sizes, a.device)
         size = sizes[index]
+        self.last = plan, index
         plan.execute(index, workspace.data_ptr() if size else 0, size, torch.cuda.current_stream(a.device).cuda_stream)
 
 

@@ -47,3 +47,24 @@ def test_gpu_arm_has_no_cpu_fallback():
     result = run_bench("--steps", "1", "--warmup", "1", timeout=300)
     assert result.returncode != 0
     assert "no CUDA device" in result.stdout
+
+
+def test_the_roofline_divisor_comes_from_the_plan():
+    """Two equal neighbouring names make a prepared form only where the first asks for more workspace than the second."""
+    import importlib.util
+
+    spec = importlib.util.spec_from_file_location("bench_under_test", REPO / "bench.py")
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+
+    class Plan:
+        entries = [("Fp32Gemm3xTf32SplitK", 9000), ("Fp32Gemm3xTf32SplitK", 4096), ("Fp32Gemm3xTf32", 0), ("Fp32Gemm3xTf32", 0), ("Fp32Gemm", 0)]
+        num_primitives = len(entries)
+
+        def primitive_name(self, index):
+            return self.entries[index][0]
+
+        def workspace_bytes(self, index):
+            return self.entries[index][1]
+
+    assert [bench.tensor_divisor(Plan(), index) for index in range(5)] == [3, 6, 6, 6, 6]
