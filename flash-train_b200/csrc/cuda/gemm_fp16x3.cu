@@ -5,7 +5,7 @@
 // when that is exact enough and leaves the launch to the TF32 kernel when it is not),
 //   a b = a_hi b_hi + (a_lo b_hi + a_hi b_lo) / 2^11,     a = a_hi + a_lo / 2^11, b likewise,
 // is three tcgen05.mma.kind::f16 products in half the tensor time of three TF32 ones, with less
-// rounding in the low parts (2^-24 against a truncation at 2^-21). And because the operands arrive
+// rounding in the low parts (2^-23 at most, to nearest, against a truncation at 2^-21). And because the operands arrive
 // split, no warp converts anything here: the conversion, which every CTA of the TF32 kernel repeats
 // for every tile, is paid once per operand element, and the tensor cores wait for TMA alone.
 //

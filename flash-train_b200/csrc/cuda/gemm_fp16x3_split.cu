@@ -4,8 +4,8 @@
 // every 16 columns of B together, are scaled by a power of two that brings their largest magnitude there to
 // [2^14, 2^15), and every scaled element x becomes
 //   hi = fp16(x),  lo = fp16((x - hi) * 2^11)      (both to nearest even)
-// so that x = hi + lo / 2^11 to within 2^-24 |x| as long as |x| >= 2^-12, i.e. for every element within
-// 2^26 of the largest; below that ("gray" elements) to within 2^-36, which is 2^-50 of the largest.
+// so that x = hi + lo / 2^11 to within 2^-23 |x| as long as |x| >= 2^-12, i.e. for every element within
+// 2^26 of the largest (1 + 2^-12 + 2^-23 is that far off: the low part is a tie); below that ("gray" elements) to within 2^-36, which is 2^-50 of the largest.
 //
 // When that is enough. An element's error e contributes e * |b| to the result: for a gray element of A at most
 // 2^-50 M_a M_b, with M the largest magnitude that either scale allows for, and with g_a gray elements in a row of A and g_b in

@@ -251,7 +251,10 @@ FTRAIN_API FTrainStatus ftrainPlanGetPrimitiveRequiredWorkspaceBytes(FTrainPlan 
  * Enqueues one Primitive on stream and returns without synchronising. The
  * calling thread's current device must be the Plan's device; workspace_bytes
  * must cover the Primitive's requirement (non-null workspace when that is
- * nonzero). The Plan, the tensors and the workspace must outlive the enqueued
+ * nonzero). One exception: a Primitive that stands in the Plan twice in a row,
+ * under one name and with two requirements, runs at its first index too when
+ * the workspace covers only the second requirement, in the slower form that
+ * the second index always runs; below that it is refused. The Plan, the tensors and the workspace must outlive the enqueued
  * work; concurrent executions of one Plan need external synchronisation.
  */
 FTRAIN_API FTrainStatus ftrainPlanExecutePrimitive(FTrainPlan plan, uint64_t primitive_index, void* workspace,

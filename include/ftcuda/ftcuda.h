@@ -52,8 +52,10 @@ enum {
     FTCUDA_GEMM_TF32X3_ROWS = 5,
     /* The prepared forms of FTCUDA_GEMM_TF32X3 and FTCUDA_GEMM_TF32X3_SPLITK: the launch splits the operands into
      * scaled FP16 pairs in the workspace (as many bytes as A and B) and multiplies those at twice the TF32 rate,
-     * with no larger error. Operands whose magnitudes spread too far within a row of A or a column of B
-     * (or are not finite) go through the TF32 family instead; the GPU decides, in the launch. */
+     * with no larger error. The GPU decides, in the launch, whether the TF32 family runs instead, after the split: where
+     * magnitudes are not finite or their largest is outside [2^-100, 2^61), and where elements more than 2^26 below the
+     * largest that shares their scale do not drown among larger ones. A scale covers 768 values along K of a row of A, and of
+     * 16 neighbouring columns of B together: a column that is small as a whole beside its neighbours counts as such elements. */
     FTCUDA_GEMM_FP16X3 = 6,
     FTCUDA_GEMM_FP16X3_SPLITK = 7,
     FTCUDA_GEMM_KERNEL_COUNT = 8,
