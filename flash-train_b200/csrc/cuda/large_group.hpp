@@ -37,21 +37,21 @@ struct OneLaunchEstimate {
     }
 };
 
-// ... and of one group's launches in the prepared form, behind those of others. 7 % off in the mean (root mean square) over the same mixes.
+// ... and of one group's launches in the prepared form, behind those of others. 8 % off in the mean (root mean square) over the same mixes.
 inline double preparedEstimate(const FtcudaGemmDesc& desc, std::uint32_t sms) {
     const std::uint64_t pairs  = sms / 2 != 0 ? sms / 2 : 1;
     const fp16x3::Geometry g   = fp16x3::chooseGeometry(desc.m, desc.n, fp16x3::divideUp(desc.k, fp16x3::kBlockK), pairs);
     const std::uint64_t items  = fp16x3::divideUp(desc.m, fp16x3::kTileM) * fp16x3::divideUp(desc.n, g.tile_n) * g.splits;
     const double waves         = static_cast<double>(fp16x3::divideUp(items, pairs));
     const double operand_bytes = 4.0 * static_cast<double>(desc.m + desc.n) * static_cast<double>(desc.k);  // read, and as many written
-    return 13.0 + waves * (4.6 + 0.61e-3 * g.blocks_per_split * fp16x3::blockCycles(g.tile_n)) + 0.574e-6 * operand_bytes;
+    return 9.3 + waves * (9.1 + 0.75e-3 * g.blocks_per_split * fp16x3::blockCycles(g.tile_n)) + 0.444e-6 * operand_bytes;
 }
 
 // Whether the large groups one after another in the prepared form, and the others in one TF32 launch, are faster than all of
 // them in that launch. What decides is how the tiles fill whole waves, of each large group and of the one launch, and whether
-// the others need a launch of their own. Measured (us, prepared / one launch): 4 x (1500 x 2048 x 2048) 226 / 285,
-// 8 x (2048 x 1024 x 2048) 336 / 380, 7 of 372 to 1861 x 4096 x 4096 1133 / 1425, but 4 x (1200 x 2816 x 1200) 228 / 170,
-// 8 x (1100 x 4096 x 1536) 669 / 496, 1500 and 130 x 2048 x 1536 115 / 72. The choice costs at most 13 % on those mixes, 3 % but for one.
+// the others need a launch of their own. Measured (us, prepared / one launch): 4 x (1500 x 2048 x 2048) 238 / 290,
+// 8 x (2048 x 1024 x 2048) 362 / 386, 7 of 372 to 1861 x 4096 x 4096 1228 / 1436, but 4 x (1200 x 2816 x 1200) 228 / 170,
+// 8 x (1100 x 4096 x 1536) 669 / 496, 1500 and 130 x 2048 x 1536 115 / 72. The choice costs at most 10 % on 72 mixes, 6 % but for one.
 inline bool preparedGroupsPay(const FtcudaGemmDesc* groups, std::uint32_t count, std::uint32_t sms) {
     OneLaunchEstimate all, others;
     double prepared = 0.0;

@@ -11,21 +11,23 @@ std::uint64_t ceilDiv(std::uint64_t x, std::uint64_t y) { return (x + y - 1) / y
 }  // namespace
 
 // The split passes over (m + n) k elements, the multiplication saves half of the tensor time of m n k, so what counts is
-// m n / (m + n). Measured (better TF32 form / prepared form, microseconds): from 600 on the prepared form is ahead as soon as
-// there is enough work (2048 x 512 x 1024 37 / 29, 1024 x 16384 x 2048 316 / 293, 2048^3 115 / 63, 4096^3 710 / 412,
-// 8192 x 4096 x 8192 2779 / 1438); at 455 and 512 only with a medium K (1024 x 4096 x 1024 59 / 51, 512 x 2048 x 4096 65 / 50,
-// but 1024^3 26 / 27, 512 x 16384 x 4096 326 / 356); below that hardly ever (512 x 4096 x 2048 51 / 60,
-// 256 x 4096 x 4096 50 / 75). Up to 45 tiles of 128 x 192 the TF32 form spreads a K of up to 4096 over clusters of three
-// CTAs or more and needs more work to be overtaken: 33.3 / 40.9 at 1040 x 2184 x 888, 35.1 / 45.3
-// at 830 x 2368 x 1152, 41.2 / 43.8 at 768 x 3264 x 1148, but 49.4 / 47.9 at 904 x 4096 x 904 and, with 48 tiles,
-// 58.4 / 44.0 at 688 x 3456 x 1384. A K under 512 was not measured.
+// m n / (m + n). Measured (TF32 form / prepared form, microseconds, B row-major): from 600 on the prepared form is ahead as soon as
+// there is enough work (2048 x 512 x 1024 29 / 27, 4096 x 512 x 704 31 / 29, 1024 x 16384 x 2048 303 / 243, 2048^3 136 / 75,
+// 4096^3 615 / 434, 8192 x 512 x 8192 448 / 297); from 450 on only with a medium K (512 x 2000 x 3800 64 / 52,
+// 512 x 1536 x 4096 52 / 39, but 512 x 16384 x 4096 307 / 299, and 326 / 356 on another GPU); below that hardly ever
+// (512 x 4096 x 2048 62 / 71, 256 x 4096 x 4096 64 / 80).
+// Up to half a wave of tiles of 128 x 192 (74) the TF32 form spreads a K of up to 4096 over a cluster for each tile and is ahead
+// (1040 x 2184 x 888 33 / 46, 752 x 2496 x 2156 45 / 53, 1152 x 1088 x 1376 29 / 35, 1152 x 2792 x 1344 49 / 55), but for a deep K
+// with 48 to 63 tiles, too many for clusters of three and too few for clusters of two to fill the SMs (688 x 3456 x 1384
+// 58 / 47, 1269 x 3584 x 896 60 / 53, 1152 x 3456 x 1216 58 / 58, and 58 / 55 with B along K). A K under 512 was not measured.
 bool preparedFormPays(const GemmShape& shape) noexcept {
     if (shape.k < 512 || shape.m < 512 || shape.n < 512) { return false; }
     const double m = static_cast<double>(shape.m), n = static_cast<double>(shape.n), products = m * n * static_cast<double>(shape.k);
     const double reuse = m * n / (m + n);
-    if (reuse >= 600.0) { return products >= 1e9; }
-    const bool few_tiles = ceilDiv(shape.m, 128) * ceilDiv(shape.n, 192) <= 45;
-    return reuse >= 450.0 && products >= (few_tiles ? 3e9 : 1.5e9) && products <= 6e9;
+    if (reuse < 450.0) { return false; }
+    const std::uint64_t tiles = ceilDiv(shape.m, 128) * ceilDiv(shape.n, 192);
+    if (tiles <= 74 && shape.k <= 4096) { return tiles >= 48 && tiles <= 63 && shape.k >= 3400; }
+    return reuse >= 600.0 ? products >= 1e9 : products >= 1.5e9 && products <= 6e9;
 }
 
 // Regime map on B200 (148 SMs; the count is queried, not assumed). The

@@ -317,13 +317,15 @@ TEST(finder_regime_map) {
 
 TEST(finder_prepared_form_where_it_was_measured_to_pay) {
     const auto pays = [](std::uint64_t m, std::uint64_t k, std::uint64_t n) { return preparedFormPays(GemmShape{m, n, k}); };
-    CHECK(pays(2048, 512, 1024) && pays(1024, 16384, 2048) && pays(4096, 4096, 4096));
-    CHECK(!pays(2048, 511, 1024) && !pays(511, 4096, 8192) && !pays(8192, 4096, 511) && !pays(1280, 600, 1280));
+    CHECK(pays(2048, 512, 1024) && pays(1024, 16384, 2048) && pays(4096, 4096, 4096) && pays(1300, 600, 1300));
+    CHECK(!pays(2048, 511, 1024) && !pays(511, 4096, 8192) && !pays(8192, 4096, 511) && !pays(1300, 550, 1300));
     // m n / (m + n) between 450 and 600: a medium K only.
-    CHECK(pays(1024, 4096, 1024) && pays(512, 2048, 4096) && !pays(1024, 1024, 1024) && !pays(512, 16384, 4096) && !pays(512, 4096, 2048));
-    // Up to 45 tiles of 128 x 192 the TF32 form's clusters are ahead for longer; 48 tiles are too many for clusters of three.
-    CHECK(!pays(1040, 2184, 888) && !pays(830, 2368, 1152) && !pays(768, 3264, 1148) && !pays(900, 2000, 910));
-    CHECK(pays(904, 4096, 904) && pays(688, 3456, 1384) && pays(1024, 1536, 1152));
+    CHECK(pays(512, 2048, 4096) && pays(512, 1536, 4096) && !pays(512, 16384, 4096) && !pays(512, 4096, 2048));
+    // Up to 74 tiles of 128 x 192 the TF32 form's clusters are ahead up to K = 4096; 48 to 63 tiles are too many for clusters of
+    // three and too few for clusters of two to fill the SMs, which a deep K makes up for the split.
+    CHECK(!pays(1040, 2184, 888) && !pays(830, 2368, 1152) && !pays(768, 3264, 1148) && !pays(900, 2000, 910) && !pays(904, 4096, 904));
+    CHECK(!pays(1152, 1088, 1376) && !pays(752, 2496, 2156) && !pays(640, 3520, 2560) && !pays(1024, 3392, 1024));
+    CHECK(pays(688, 3456, 1384) && pays(1269, 3584, 896) && pays(1024, 4096, 1024) && pays(715, 4928, 1408));
 }
 
 TEST(builtin_gemm_engine_is_registered) {
