@@ -21,10 +21,12 @@
 // Tensor memory holds two accumulators, 512 columns in all: X, the two cross products, issued by warp 1, and H, a_hi b_hi,
 // issued by warp 2. Both are read at the end of every slab of K (768, the split's unit of scaling), multiplied by
 // the slab's powers of two (addScaled) and added up in registers, to nearest. The tensor core's own FP32
-// additions truncate, so for a small K H is read more often than that (chunkBlocks); X is 2^11 times smaller
-// in effect. With an issuer each, one accumulator is read while products go to the other, and what a single thread does
+// additions truncate, so below K = 22500 H is read more often than that (chunkBlocks); X is 2^11 times smaller
+// in effect. A reading of H leaves the tensor pipe idle for about 1000 cycles, nearly all of it the way through the barriers:
+// without loads or additions in the drain it costs the same (timing build, 4096^3: 349 us with one per slab, 374 with three, 367
+// with three empty ones). Holding the cross products' issuer back so that H's last products of a sum go first gave 1 %, or lost. With an issuer each, one accumulator is read while products go to the other, and what a single thread does
 // between two K blocks -- barriers, descriptors -- no longer leaves the tensor pipe idle (one issuer for both:
-// 440 us instead of 388 at 4096^3, 187 instead of 154 at 2048 x 4096 x 3072). Rings of their own for the high and
+// 440 us instead of 388 at 4096^3, 187 instead of 154 at 2048 x 4096 x 3072, each with one reading per slab). Rings of their own for the high and
 // the low parts, with H held one block behind X, were not faster (398 to 421 us).
 //
 // Shared memory is the resource next to the tensor pipe: operand fetches and TMA writes take 106 of its 128 bytes a
@@ -32,9 +34,8 @@
 // the results go to memory straight from registers, 32 bytes a thread and store: 9400 cycles a tile, 15000 in pieces of
 // 16 bytes, 12000 turned in shared memory first (and the MMAs slower meanwhile).
 //
-// Measured, the whole launch with its split, TF32 form / this one in microseconds: 16384 x 4096 x 14336 8850 / 4600 (up
-// to 426 TFLOP/s; what bounds it is the power limit: the products alone run at 0.91 of the measured dense BF16
-// rate), 8192 x 4096 x 8192 2780 / 1440, 4096^3 710 / 400, 2048^3 115 / 63, 1024 x 1024 x 4096 83 / 39.
+// Measured, the whole launch with its split, TF32 form / this one in microseconds: 16384 x 4096 x 14336 9000 / 5100 (398
+// to 415 TFLOP/s in bursts; power-limited), 8192 x 4096 x 8192 2530 / 1440, 4096^3 640 / 426, 2048^3 132 / 70, 1024 x 1024 x 4096 76 / 40.
 //
 // Every wait is bounded, as in the other kernels (ptx.cuh).
 #include <cuda.h>
